@@ -639,9 +639,9 @@ struct Session {
         reset();
         set_window(cfg->tstart, cfg->tstart + cfg->tstep * (float)k.maxgate);   // first gate group
 
+        k.seed_mode = seeding_mode();       // before the launch shape: the kernel variant depends on it
         configure_launch(cfg);
 
-        k.seed_mode = seeding_mode();
         if (k.seed_mode == 1) {
             // the thread count MCX's autopilot picks on this device (src/mcx_core.cu:2554-2608,
             // 2688-2695, 3050-3053), or the user's nthread/nblocksize without autopilot

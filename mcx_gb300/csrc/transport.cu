@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <cstddef>
 #include <cstdint>
 #include "transport.cuh"
 
@@ -1554,6 +1555,8 @@ __global__ void __launch_bounds__(256, MINB) transport_kernel(const __grid_const
     }
 }
 
+#include "transport_lean.cuh"
+
 // Roofline probe: fire-and-forget FP32 reductions to addresses spread over `n` floats (a hash of
 // the thread and iteration), the operation the transport kernel's deposits reduce to.
 __global__ void atomic_probe_kernel(float* buf, unsigned n, int iters) {
@@ -1604,7 +1607,14 @@ __global__ void merge_kernel(float* __restrict__ out, const float* __restrict__ 
 
 }  // namespace
 
+// The plain path (transport_lean.cuh): what its kernel leaves out must be off.  No photon reaches
+// gscatter scattering events when that is past the step cap (checked every 1024 steps).
+static bool lean_path(const KParams& p) {
+    return p.seed_mode == 0 && !p.field64 && p.save2pt && !(p.minenergy > 0.f) && p.gscatter > (float)p.step_cap + 2048.f;
+}
+
 size_t transport_smem_bytes(const KParams& p, int block, bool savedet) {
+    if (transport_mode(p) >= kLeanPencil) return lean_smem_bytes(p, savedet);
     size_t b = sizeof(float4) * (size_t)p.medianum;
     b += (2 * sizeof(unsigned long long) + sizeof(int) + 3 * sizeof(unsigned)) * (size_t)(block / 32);
     b += 4 * sizeof(unsigned) * (size_t)block;
@@ -1631,7 +1641,8 @@ int transport_mode(const KParams& p) {
     if (p.replay || p.saveseed || p.outputtype > kOutEnergy || p.traj || p.polarized || p.saveref || p.srcnum > 1 ||
         p.nphase > 2 || p.nangle > 0 || p.nextra > 0)
         return 2;
-    return (p.srctype != kSrcPencil) ? 1 : 0;
+    const int area = (p.srctype != kSrcPencil) ? 1 : 0;
+    return lean_path(p) ? kLeanPencil + area : area;
 }
 
 template <int M, int K>
@@ -1640,9 +1651,17 @@ static const void* pick_flags(bool reflect, bool savedet) {
     return savedet ? kernel_ptr<false, true, M, K>() : kernel_ptr<false, false, M, K>();
 }
 
+template <bool AREA, int M>
+static const void* pick_lean(bool reflect, bool savedet) {
+    if (reflect) return savedet ? (const void*)lean_kernel<true, true, AREA, M> : (const void*)lean_kernel<true, false, AREA, M>;
+    return savedet ? (const void*)lean_kernel<false, true, AREA, M> : (const void*)lean_kernel<false, false, AREA, M>;
+}
+
 // The pencil variants run at 4 CTAs of 256 per SM (64 registers) unless the tuner asks for 3;
 // the variants with the general launch need more registers and run at 3 (80 registers).
 static const void* pick(bool reflect, bool savedet, int mode) {
+    if (mode == kLeanArea) return pick_lean<true, 3>(reflect, savedet);
+    if (mode == kLeanPencil) return pick_lean<false, 4>(reflect, savedet);
     if (mode == 4) return pick_flags<3, 4>(reflect, savedet);
     if (mode == 3) return pick_flags<3, 3>(reflect, savedet);
     if (mode == 2) return pick_flags<3, 2>(reflect, savedet);
@@ -1698,6 +1717,7 @@ static KParams finalize(const KParams& in) {
     p.d_fnx = (float)p.nx; p.d_fny = (float)p.ny; p.d_fnz = (float)p.nz;
     p.d_tx0 = (float)p.tx0; p.d_ty0 = (float)p.ty0; p.d_tz0 = (float)p.tz0;
     p.d_tx1 = (float)(p.tx0 + p.tnx); p.d_ty1 = (float)(p.ty0 + p.tny); p.d_tz1 = (float)(p.tz0 + p.tnz);
+    p.d_tnx = (float)p.tnx; p.d_tny = (float)p.tny; p.d_tnz = (float)p.tnz;
     p.d_n0 = p.prop[0].w;
     p.d_gscat = (p.gscatter >= 2147483647.f) ? 2147483647 : (int)p.gscatter;
     p.d_nwork = (p.seed_mode == 1 && !p.replay) ? (unsigned long long)p.mcx_streams : p.nphoton;
@@ -1717,6 +1737,8 @@ cudaError_t launch_transport(const KParams& in, bool reflect, bool savedet, int 
     // need: whole-chunk reservations would leave some warps with two rounds of photons while
     // others have none, and the launch would end on their tail
     if (p.d_nwork < (unsigned long long)grid * (unsigned long long)block * 16ull) p.chunk = 1;
+    // the caller sized the shared memory for the variant of its parameters: never launch another's
+    if (smem_bytes < transport_smem_bytes(p, block, savedet)) return cudaErrorInvalidValue;
     const void* k = pick(reflect, savedet, transport_mode(p));
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
     if (e != cudaSuccess) return e;

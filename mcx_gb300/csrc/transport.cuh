@@ -170,6 +170,7 @@ struct KParams {
     float d_bin_a, d_bin_b;         // gate index = floor(t * d_bin_a - d_bin_b)
     float d_fnx, d_fny, d_fnz;      // dimensions as floats
     float d_tx0, d_ty0, d_tz0, d_tx1, d_ty1, d_tz1;   // tile box as floats
+    float d_tnx, d_tny, d_tnz;      // its sizes as floats
     float d_n0;                     // refractive index of medium 0
     int d_gscat;                    // gscatter as an integer threshold
     unsigned long long d_nwork;     // work items in the pool: photons, or MCX streams
@@ -203,7 +204,9 @@ int transport_variant();
 size_t transport_smem_bytes(const KParams& p, int block, bool savedet);
 // Kernel variant of a parameter set: 0 = pencil beam with flux/fluence/energy output, 1 = other
 // source shapes sampled per photon, 2 = replay, seed saving or the replay / path-length outputs,
-// 3 = everything of 2 on a per-voxel media format.
+// 3 = everything of 2 on a per-voxel media format, 4 = split voxels; kLeanPencil / kLeanArea = 0 / 1
+// on the plain path (transport_lean.cuh).
+constexpr int kLeanPencil = 8, kLeanArea = 9;
 int transport_mode(const KParams& p);
 bool transport_general(const KParams& p);
 // Occupancy-derived CTAs per SM for the chosen variant.
