@@ -7,7 +7,8 @@
 // bf16 [Cout][taps][Cin] with tap = dz*9 + dy*3 + dx; master weights, gradients and Adam moments
 // are fp32 in the same order.
 //
-// Convolutions are implicit GEMMs on the BF16 tensor cores (mma.sync m16n8k16, fp32 accumulate):
+// Convolutions are implicit GEMMs on the BF16 tensor cores, fp32 accumulate: the 3x3x3 ones forward and as data
+// gradients on tcgen05 (conv3_roll.cuh), the weight gradient and what that kernel does not take on mma.sync m16n8k16:
 //   forward   Y[v, co]  = sum_{t, ci} X[v + off(t), ci] * W[co, t, ci]      (M = voxels, N = Cout)
 //   data grad dX[v, ci] = sum_{t, co} dY[v + off(t), co] * W[co, 26-t, ci] (the forward kernel run
 //             on the flipped, transposed copy of W that the optimiser writes beside the weights)
@@ -106,7 +107,7 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N) conv_fwd_kernel(
     constexpr int A_IT = BM * CPR / THREADS;
     static_assert(NI % 2 == 0 && MI >= 1 && A_IT >= 1 && (BM * CPR) % THREADS == 0 && THREADS % CPR == 0, "tile shape");
 
-    extern __shared__ __align__(128) unsigned char dyn_smem[];
+    extern __shared__ __align__(1024) unsigned char dyn_smem[];
     bf16* sm = reinterpret_cast<bf16*>(dyn_smem);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(128) conv3_halo_kernel(const bf16* __restrict_
     constexpr int WARPS_M = 4, WM = BM / WARPS_M, MI = WM / 16, NI = BN / 8;
     static_assert(NI % 2 == 0 && MI == 2, "tile shape");
     constexpr int ROWB = 32;                     // bytes per halo / weight row (16 channels)
-    extern __shared__ __align__(128) unsigned char dyn_smem[];
+    extern __shared__ __align__(1024) unsigned char dyn_smem[];
     unsigned char* sh = dyn_smem;                // [HV][32 B]
     unsigned char* sw = dyn_smem + HV * ROWB;    // [27][BN][32 B]
 
@@ -403,26 +404,9 @@ __global__ void __launch_bounds__(128) conv3_halo_kernel(const bf16* __restrict_
 }
 
 // ---------------------------------------------------------------------------------------------
-// 3x3x3 convolution for narrow outputs (BN = 16 or 32 channels) on the fifth-generation tensor
-// cores: tcgen05.mma (cta_group::1, kind::f16, BF16 operands from shared memory, FP32 accumulator
-// in tensor memory), issued by one thread, with the input halos brought in by TMA.  A tile is two
-// z-planes of 16 y rows x 8 x voxels; each plane is one M = 128 MMA, whose eight-voxel rows are
-// a uniform stride apart in the halo.  Per 16-channel slice of the input, the 4 x 18 x 10 halo
-// around the tile lands as two 8-channel planes of 16-byte rows, and every tap's A operand is the same halo
-// seen through a descriptor whose start moves by the tap's row offset: K-major, no swizzle, core
-// matrices of 8 consecutive rows (8 consecutive x), the 8-row groups HX rows apart (stride byte
-// offset), the second 8 channels one plane further on (leading byte offset).  The weights of a
-// slice's 27 taps sit in shared memory as [tap][8-channel half][co] 16-byte rows.  Each slice is
-// 27 MMAs of 128 x BN x 16 into one accumulator.  The epilogue reads the accumulator rows (TMEM
-// lane = voxel) with tcgen05.ld, adds bias, applies ReLU and the mask, and stores bf16.  Every
-// wait is bounded: a wait that gives up sets g_dn_fault, and the CTA still releases its tensor
-// memory and returns.
+// Fifth-generation tensor cores (tcgen05): descriptors, bounded waits, tensor-memory loads.  A wait
+// that gives up sets g_dn_fault, which mcxg_dn_check reports.
 __device__ unsigned g_dn_fault;
-
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
-}
 
 // kind::f16 instruction descriptor: FP32 accumulator, BF16 A and B, both K-major, M = 128, N = n.
 __host__ __device__ constexpr uint32_t umma_idesc_bf16(int n) {
@@ -453,244 +437,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
-template <int BN>
-struct TcConvShape {
-    static constexpr int TZ = 2, TY = 16, TX = 8;                         // two z-planes of 128 voxels
-    static constexpr int HZ = TZ + 2, HY = TY + 2, HX = TX + 2, HV = HZ * HY * HX;   // 720 halo rows
-    static constexpr int PLANE = HV * 16;                                 // 11520 B, a multiple of 128
-    static constexpr int HALO = 2 * PLANE;                                // one stage: 16 channels
-    static constexpr int HALO_BYTES = 2 * HV * 16;                        // bytes the two copies bring
-    static constexpr int WTAP = 2 * BN * 16;                              // one tap's weights
-    static constexpr int WSLICE = 27 * WTAP;                              // one 16-channel slice
-    static constexpr int MAX_STAGES = 4;
-};
-
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-// Warp roles: warps 0-3 drain the accumulators (warp w reads TMEM lanes 32w..32w+31, the voxels of
-// its quarter of the tile), warp 4 issues the TMA copies of the halos, warp 5 issues the MMAs.
-// The CTA is persistent: it loads the weights of every input slice once, then walks its tiles
-// (blockIdx.x, + gridDim.x, ...) as a sequence of (tile, slice) items.  Each item is one halo: two
-// TMA tile copies (channels c..c+7 and c+8..c+15) of a 4 x 18 x 10 voxel box of the channels-last
-// activations, described by a 5-D tensor map (channel, x, y, z, volume) whose out-of-volume rows
-// arrive as zeros; the box lands as 720 rows of 16 bytes, x fastest, which is the A operand's
-// canonical no-swizzle K-major layout.  Halos cycle through `stages` buffers (full barriers: the
-// copies landed; empty barriers: the MMAs that read the buffer finished), and tiles through two
-// TMEM accumulators (accfull: a tile's MMAs finished; accempty: its epilogue has read it), so
-// copies, MMAs and epilogues of neighbouring items overlap.
-template <int BN>
-__global__ void __launch_bounds__(192) conv3_tc_kernel(const __grid_constant__ CUtensorMap tmap,
-                                                       const bf16* __restrict__ wt, const float* __restrict__ bias,
-                                                       const bf16* __restrict__ mask, bf16* __restrict__ y, Geo g,
-                                                       int cin, int cout, int relu, int tiles_x, int tiles_y,
-                                                       int ntiles, int stages) {
-    using S = TcConvShape<BN>;
-    constexpr uint32_t TMEM_COLS = 4 * BN;          // two tiles in flight x two z-planes of BN columns
-    static_assert(BN == 16 || BN == 32, "tile width");
-    static_assert(S::WSLICE % 128 == 0 && S::PLANE % 128 == 0 && S::PLANE >= S::HV * 16, "TMA / UMMA alignment");
-    extern __shared__ __align__(1024) unsigned char dyn_smem[];
-    __shared__ __align__(8) uint64_t s_bar[2 * S::MAX_STAGES + 4];
-    __shared__ uint32_t s_tmem;
-
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int slices = cin / 16;
-    const int n0 = blockIdx.y * BN;
-    // weights first, then the halo stages (the weight block is a multiple of 128 bytes)
-    const uint32_t sw_addr = smem_addr(dyn_smem);
-    const uint32_t sh_addr = sw_addr + slices * S::WSLICE;
-    const uint32_t full0 = smem_addr(&s_bar[0]), empty0 = full0 + 8 * S::MAX_STAGES;
-    const uint32_t accfull0 = empty0 + 8 * S::MAX_STAGES, accempty0 = accfull0 + 16;
-    const int my_tiles = ntiles > (int)blockIdx.x ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    const int items = my_tiles * slices;
-
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&s_tmem)),
-                     "n"(TMEM_COLS));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
-    }
-    if (tid == 0) {
-        for (int i = 0; i < 2 * S::MAX_STAGES + 2; ++i)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(full0 + 8 * i));
-        for (int i = 0; i < 2; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;\n" ::"r"(accempty0 + 8 * i));
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    // the weights of every slice, once: [slice][tap][8-channel half][co] rows of 16 bytes
-    for (int q = tid; q < slices * 27 * 2 * BN; q += 192) {
-        const int co = q % BN, r = q / BN, kb = r & 1, t = (r >> 1) % 27, sl = (r >> 1) / 27;
-        const bf16* p = wt + ((long long)(n0 + co) * 27 + t) * cin + sl * 16 + kb * 8;
-        cp_async16(sw_addr + sl * S::WSLICE + t * S::WTAP + kb * BN * 16 + co * 16, p, true);
-    }
-    cp_commit();
-    cp_wait<0>();
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = s_tmem;
-
-    struct TileAt {
-        int x0, y0, z0, n;
-    };
-    auto tile_at = [&](int j) {
-        int tile = (int)blockIdx.x + j * (int)gridDim.x;
-        TileAt r;
-        r.x0 = (tile % tiles_x) * S::TX;
-        tile /= tiles_x;
-        r.y0 = (tile % tiles_y) * S::TY;
-        tile /= tiles_y;
-        const int tz = (g.d + S::TZ - 1) / S::TZ;
-        r.z0 = (tile % tz) * S::TZ;
-        r.n = tile / tz;
-        return r;
-    };
-
-    bool fault = false;
-    if (warp == 4) {
-        // ---- producer: TMA halo copies ----------------------------------------------------------
-        if (lane == 0) {
-            const uint64_t map = reinterpret_cast<uint64_t>(&tmap);
-            for (int k = 0; k < items; ++k) {
-                const int b = k % stages;
-                if (k >= stages && !mbar_wait(empty0 + 8 * b, ((k / stages) - 1) & 1)) {
-                    fault = true;
-                    break;
-                }
-                const TileAt T = tile_at(k / slices);
-                const int c0 = (k % slices) * 16;
-                const uint32_t bar = full0 + 8 * b, dst = sh_addr + b * S::HALO;
-                mbar_expect_tx(bar, S::HALO_BYTES);
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    asm volatile(
-                        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
-                        "%5, %6}], [%7];\n" ::"r"(dst + h * S::PLANE),
-                        "l"(map), "r"(c0 + 8 * h), "r"(T.x0 - 1), "r"(T.y0 - 1), "r"(T.z0 - 1), "r"(T.n), "r"(bar)
-                        : "memory");
-            }
-        }
-        __syncwarp();
-    } else if (warp == 5) {
-        // ---- MMA issue: one thread --------------------------------------------------------------
-        if (lane == 0) {
-            for (int k = 0; k < items; ++k) {
-                const int j = k / slices, sl = k - j * slices, b = k % stages;
-                if (!mbar_wait(full0 + 8 * b, (k / stages) & 1)) {
-                    fault = true;
-                    break;
-                }
-                if (sl == 0 && j >= 2 && !mbar_wait(accempty0 + 8 * (j & 1), ((j - 2) >> 1) & 1)) {
-                    fault = true;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint32_t d = tmem + (uint32_t)((j & 1) * 2 * BN);
-                // descriptors of tap 0; a tap (and the second z-plane, one halo plane further on)
-                // moves the start address (bits 0-13, in 16-byte units) by a constant, so the 54 MMAs
-                // issue back to back; both planes share the tap's weights
-                const uint64_t ad0 = umma_desc(sh_addr + b * S::HALO, S::PLANE, S::HX * 16);
-                const uint64_t bd0 = umma_desc(sw_addr + sl * S::WSLICE, BN * 16, 128);
-#pragma unroll
-                for (int t = 0; t < 27; ++t) {
-                    const uint64_t bd = bd0 + (uint64_t)(t * S::WTAP >> 4);
-                    const uint32_t accum = (sl > 0 || t > 0) ? 1u : 0u;
-#pragma unroll
-                    for (int zp = 0; zp < S::TZ; ++zp) {
-                        const uint64_t ad =
-                            ad0 + (uint64_t)((((t / 9 + zp) * S::HY + (t / 3) % 3) * S::HX + t % 3) * 16 >> 4);
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d + zp * BN),
-                            "l"(ad), "l"(bd), "n"(umma_idesc_bf16(BN)), "r"(accum)
-                            : "memory");
-                    }
-                }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                                 empty0 + 8 * b)
-                             : "memory");
-                if (sl == slices - 1)
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                                     accfull0 + 8 * (j & 1))
-                                 : "memory");
-            }
-        }
-        __syncwarp();
-    } else {
-        // ---- epilogue: warps 0-3 -------------------------------------------------------------------
-        for (int j = 0; j < my_tiles; ++j) {
-            const bool ok = mbar_wait(accfull0 + 8 * (j & 1), (j >> 1) & 1);
-            if (!__all_sync(0xffffffffu, ok)) {
-                fault = true;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const TileAt T = tile_at(j);
-            const int r = warp * 32 + lane;             // accumulator row = TMEM lane = voxel of a plane
-            const int yy = T.y0 + (r >> 3), xx = T.x0 + (r & 7);
-            uint32_t v[S::TZ][BN];
-#pragma unroll
-            for (int zp = 0; zp < S::TZ; ++zp)
-#pragma unroll
-                for (int c0 = 0; c0 < BN; c0 += 16)
-                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((j & 1) * 2 * BN + zp * BN + c0),
-                              *reinterpret_cast<uint32_t(*)[16]>(&v[zp][c0]));
-            // the accumulators are free again once every lane of the four warps has read them
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(accempty0 + 8 * (j & 1));
-#pragma unroll
-            for (int zp = 0; zp < S::TZ; ++zp) {
-                if (yy >= g.h || xx >= g.w || T.z0 + zp >= g.d) continue;
-                const long long vo = (((long long)T.n * g.d + T.z0 + zp) * g.h + yy) * g.w + xx;
-#pragma unroll
-                for (int c0 = 0; c0 < BN; c0 += 16) {
-                    uint32_t pk[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        float a = __uint_as_float(v[zp][c0 + 2 * e]), bb = __uint_as_float(v[zp][c0 + 2 * e + 1]);
-                        if (bias) {
-                            a += bias[n0 + c0 + 2 * e];
-                            bb += bias[n0 + c0 + 2 * e + 1];
-                        }
-                        if (relu) {
-                            a = fmaxf(a, 0.f);
-                            bb = fmaxf(bb, 0.f);
-                        }
-                        __nv_bfloat162 h2 = __floats2bfloat162_rn(a, bb);
-                        pk[e] = *reinterpret_cast<uint32_t*>(&h2);
-                    }
-                    const long long o = vo * cout + n0 + c0;
-#pragma unroll
-                    for (int hlf = 0; hlf < 2; ++hlf) {
-                        uint4 val = make_uint4(pk[4 * hlf], pk[4 * hlf + 1], pk[4 * hlf + 2], pk[4 * hlf + 3]);
-                        if (mask) {
-                            uint4 mk = *reinterpret_cast<const uint4*>(mask + o + 8 * hlf);
-                            uint32_t* pv = reinterpret_cast<uint32_t*>(&val);
-                            const uint32_t* pm = reinterpret_cast<const uint32_t*>(&mk);
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                uint32_t lo = (pm[e] & 0xFFFFu), hi = pm[e] >> 16;
-                                uint32_t keep = ((lo & 0x8000u) == 0 && lo != 0 ? 0xFFFFu : 0u) |
-                                                ((hi & 0x8000u) == 0 && hi != 0 ? 0xFFFF0000u : 0u);
-                                pv[e] &= keep;
-                            }
-                        }
-                        *reinterpret_cast<uint4*>(y + o + 8 * hlf) = val;
-                    }
-                }
-            }
-        }
-    }
-    if (fault && lane == 0) atomicOr(&g_dn_fault, 1u);
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(TMEM_COLS));
-}
+#include "conv3_roll.cuh"
 
 // ---------------------------------------------------------------------------------------------
 // Weight gradient: dW[co, n] += sum_v dY[v, co] * X[v + off(t), ci], n = t*Cin + ci, over the
@@ -710,7 +460,7 @@ __global__ void __launch_bounds__(128) conv_wgrad_kernel(const bf16* __restrict_
     constexpr int STAGE = A_ELEMS + B_ELEMS;
     static_assert(NI % 2 == 0 && MI >= 1, "tile shape");
 
-    extern __shared__ __align__(128) unsigned char dyn_smem[];
+    extern __shared__ __align__(1024) unsigned char dyn_smem[];
     bf16* sm = reinterpret_cast<bf16*>(dyn_smem);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1216,55 +966,113 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-template <int BN>
-int conv3_tc_launch(const bf16* x, const bf16* w, const float* bias, const bf16* mask, bf16* y, Geo g, int cin,
-                    int cout, int relu, cudaStream_t st) {
-    using S = TcConvShape<BN>;
-    if (!aligned16(x)) return fail("conv: the input must be 16-byte aligned");
+// Shared memory of conv3_roll_kernel beside its barriers.
+constexpr int kRollSmem = 225 * 1024;
+
+// Launch of conv3_roll_kernel for BN output channels a block (BN divides cout).
+template <int BN, bool TAPS>
+int conv3_roll_launch(const bf16* x, const bf16* w, const float* bias, const bf16* mask, bf16* y, Geo g, int cin,
+                      int cout, int relu, int sms, cudaStream_t st) {
+    using S = RollShape<BN>;
     auto encode = tensor_map_encoder();
     if (!encode) return fail("conv: cuTensorMapEncodeTiled is not available");
-    // activations [nvol][d][h][w][cin] as a 5-D tensor (channel fastest) with a 8 x 10 x 18 x 4 x 1 box
-    CUtensorMap tmap;
-    const cuuint64_t dims[5] = {(cuuint64_t)cin, (cuuint64_t)g.w, (cuuint64_t)g.h, (cuuint64_t)g.d, (cuuint64_t)g.nvol};
-    const cuuint64_t strides[4] = {(cuuint64_t)cin * 2, (cuuint64_t)g.w * cin * 2, (cuuint64_t)g.h * g.w * cin * 2,
-                                   (cuuint64_t)g.d * g.h * g.w * cin * 2};
-    const cuuint32_t box[5] = {8, (cuuint32_t)S::HX, (cuuint32_t)S::HY, (cuuint32_t)S::HZ, 1};
-    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    if (encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16*>(x), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return fail("conv: cuTensorMapEncodeTiled rejected the activation layout");
-    const int wbytes = (cin / 16) * S::WSLICE;
-    const int limit = 227 * 1024;
-    int stages = (limit - wbytes) / S::HALO;
-    if (stages > S::MAX_STAGES) stages = S::MAX_STAGES;
-    if (stages < 2) return fail("conv: weights of this layer do not fit in shared memory");
-    // two CTAs per SM hide each other's waits better than a fourth halo stage does
-    while (stages > 3 && 2 * (wbytes + stages * S::HALO + 2048) > 228 * 1024) --stages;
-    const int smem = wbytes + stages * S::HALO;
-    auto kern = conv3_tc_kernel<BN>;
-    static int attr = 0;
-    if (smem > attr) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        attr = smem;
+    CUtensorMap xmap, wmap;
+    {
+        // activations [nvol][d][h][w][cin], a box of 16 channels of two halo planes (one in tap-major order)
+        const cuuint64_t dims[5] = {(cuuint64_t)cin, (cuuint64_t)g.w, (cuuint64_t)g.h, (cuuint64_t)g.d, (cuuint64_t)g.nvol};
+        const cuuint64_t strides[4] = {(cuuint64_t)cin * 2, (cuuint64_t)g.w * cin * 2, (cuuint64_t)g.h * g.w * cin * 2,
+                                       (cuuint64_t)g.d * g.h * g.w * cin * 2};
+        const cuuint32_t box[5] = {16, (cuuint32_t)S::HX, (cuuint32_t)S::HY, TAPS ? 1u : 2u, 1};
+        const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+        if (encode(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16*>(x), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return fail("conv: cuTensorMapEncodeTiled rejected the activation layout");
+    }
+    {
+        // weights [cout][dz][dydx][cin] seen as (ci, co, dz, dydx): a box of a slice lands as the rows
+        // (dydx, dz, co) that the MMAs of N = 3 BN read
+        const cuuint64_t dims[4] = {(cuuint64_t)cin, (cuuint64_t)cout, 3, 9};
+        const cuuint64_t strides[3] = {(cuuint64_t)27 * cin * 2, (cuuint64_t)9 * cin * 2, (cuuint64_t)cin * 2};
+        const cuuint32_t box[4] = {16, (cuuint32_t)BN, 3, 9};
+        const cuuint32_t estr[4] = {1, 1, 1, 1};
+        if (encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(w), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return fail("conv: cuTensorMapEncodeTiled rejected the weight layout");
     }
     const int tx = (g.w + S::TX - 1) / S::TX, ty = (g.h + S::TY - 1) / S::TY;
-    const long long tiles = (long long)g.nvol * ((g.d + S::TZ - 1) / S::TZ) * tx * ty;
-    if (tiles >= (1LL << 31)) return fail("conv: too many tiles");
-    // persistent CTAs: as many as shared memory lets stay resident on every SM
+    const long long planes = (long long)(cout / BN) * g.nvol * tx * ty * g.d;
+    if (planes >= (1LL << 31)) return fail("conv: too many tiles");
+    const int slices = cin / 16, stage = TAPS ? slices * S::ENTRY : S::STAGE;
+    // all slices' weights beside the halo stages (tap-major: always; else beside at least four, or a ring of two)
+    int wbufs = slices;
+    if (!TAPS && (slices > S::MAX_W || slices * S::WSLICE + 4 * stage > kRollSmem)) wbufs = 2;
+    int stages = (kRollSmem - wbufs * S::WSLICE) / stage;
+    if (stages > (TAPS ? S::MAX_STAGES : 8)) stages = TAPS ? S::MAX_STAGES : 8;
+    // a CTA takes all of an SM's tensor memory: more than half its shared memory keeps a second one away
+    int smem = wbufs * S::WSLICE + stages * stage;
+    if (smem < 120 * 1024) smem = 120 * 1024;
+    auto kern = conv3_roll_kernel<BN, TAPS>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const int grid = (int)(planes < sms ? planes : sms);
+    const int chunk = TAPS || slices == 1 ? g.d : S::R;
+    const bool wide = ((reinterpret_cast<uintptr_t>(y)) & 31u) == 0;
+    kern<<<grid, 320, smem, st>>>(xmap, wmap, bias, mask, y, g, cin, cout, relu, tx, ty, (int)planes, chunk, stages, wbufs,
+                                  wide ? 1 : 0);
+    return launched();
+}
+
+// Estimated cycles of a CTA's run of conv3_roll_kernel<bn>: its MMAs (the larger of 3027 multiply-adds and 80 operand
+// bytes a cycle, the rates the kernel measured at N = 192 and below) or its copies (a row a cycle), over the planes
+// of its run and two halo planes per piece.  Negative where the tap-major order does not fit in shared memory.
+double roll_cost(const Geo& g, int cin, int cout, int bn, bool taps, int sms) {
+    const int slices = cin / 16, R = 512 / bn;
+    const double planes = (double)(cout / bn) * g.nvol * ((g.w + 7) / 8) * ((g.h + 15) / 16) * g.d;
+    const double run = ceil(planes / (planes < sms ? planes : sms));
+    const double piece = (taps || slices == 1 || g.d < R) ? g.d : R;
+    const double pieces = run > piece ? ceil(run / piece) : 1.0;
+    const double halo = run + 2.0 * pieces;
+    const int n = (int)(run < 3 ? run : 3) * bn;
+    const double rate = 128.0 * 16.0 * n / 3027.0, read = 32.0 * (128 + n) / 80.0;
+    const double math = 9.0 * slices * halo * (rate > read ? rate : read);
+    if (taps) {
+        // the weights come first; two halo planes at least, so that one is copied while the other is read
+        if (slices > RollShape<16>::MAX_W || kRollSmem - slices * 27 * bn * 32 < 2 * slices * RollShape<16>::ENTRY) return -1.0;
+        return math + 27.0 * bn * slices;
+    }
+    const double copies = slices * (180.0 * halo + 27.0 * bn * pieces);
+    return math > copies ? math : copies;
+}
+
+// `taps`: the tap-major order.  Returns 1 where no block width fits it.
+int conv3_roll_dispatch(const bf16* x, const bf16* w, const float* bias, const bf16* mask, bf16* y, Geo g, int cin,
+                        int cout, int relu, bool taps, cudaStream_t st) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int per_sm = (228 * 1024) / (smem + 2048);
-    if (per_sm > 8) per_sm = 8;
-    if (per_sm < 1) per_sm = 1;
-    const int ny = cout / BN;
-    long long grid = (long long)sms * per_sm / ny;
-    if (grid < 1) grid = 1;
-    if (grid > tiles) grid = tiles;
-    kern<<<dim3((unsigned)grid, (unsigned)ny), 192, smem, st>>>(tmap, w, bias, mask, y, g, cin, cout, relu, tx, ty,
-                                                               (int)tiles, stages);
-    return launched();
+    int best = 0;
+    double cost = 0.0;
+    for (int bn : {16, 32, 48, 64}) {
+        if (cout % bn) continue;
+        const double c = roll_cost(g, cin, cout, bn, taps, sms);
+        if (c >= 0.0 && (!best || c < cost)) {
+            best = bn;
+            cost = c;
+        }
+    }
+#define ROLL(BN)                                                                                            \
+    case BN:                                                                                                \
+        return taps ? conv3_roll_launch<BN, true>(x, w, bias, mask, y, g, cin, cout, relu, sms, st)         \
+                    : conv3_roll_launch<BN, false>(x, w, bias, mask, y, g, cin, cout, relu, sms, st)
+    switch (best) {
+        ROLL(64);
+        ROLL(48);
+        ROLL(32);
+        ROLL(16);
+        default: return 1;
+    }
+#undef ROLL
 }
 
 // Narrow 3x3x3 layers run on tcgen05 unless MCXG_DN_MMA_SYNC=1 selects the warp-level mma.sync
@@ -1281,9 +1089,11 @@ bool use_tcgen05() {
 int conv_fwd_dispatch(const bf16* x, const bf16* w, const float* bias, const bf16* mask, bf16* y, Geo g, int cin,
                       int cout, int taps, int relu, cudaStream_t st) {
     if (use_tcgen05() && taps == 27 && cin % 16 == 0) {
-        if (cout % 32 == 0 && cout / 32 <= 3 && cout % 64 != 0)
-            return conv3_tc_launch<32>(x, w, bias, mask, y, g, cin, cout, relu, st);
-        if (cout % 32 != 0) return conv3_tc_launch<16>(x, w, bias, mask, y, g, cin, cout, relu, st);
+        // 16, 32, 48, 80, 96 .. outputs sum slice by slice, the wider layers tap by tap: the orders of the kernels
+        // this one stands in for, kept because a whole network's bf16 roundings follow from them
+        const bool narrow = cout % 32 != 0 || (cout / 32 <= 3 && cout % 64 != 0);
+        const int rc = conv3_roll_dispatch(x, w, bias, mask, y, g, cin, cout, relu, !narrow, st);
+        if (rc != 1) return rc;
     }
     // narrow 3x3x3 layers: halo tiles (each input voxel loaded once per tile, not once per tap)
     if (taps == 27 && cin % 16 == 0 && cout % 32 == 0 && cout / 32 <= 3 && cout % 64 != 0)
