@@ -35,6 +35,12 @@ int  mcxg_validatecfg(Config* cfg);
  * Replaces mcx_maskdet, src/mcx_utils.c:4214-4340 (label media). */
 void mcxg_maskdet(Config* cfg);
 
+/* Integer labels of 1, 2, 4 or 8 bytes in C order [x][y][z], converted to 32 bits as C converts them, into
+ * dst in MCX's x-fastest order (what MCX does for isrowmajor input, src/mcx_utils.c:1620-1631, without the
+ * intermediate volume).  0, or -4 for a null pointer, an empty volume or another item size. */
+int  mcxg_widen_labels(const void* src, int itemsize, int is_signed, unsigned int nx, unsigned int ny, unsigned int nz,
+                       uint32_t* dst);
+
 /* ---- Errors ------------------------------------------------------------------------------ */
 
 /* When no front-end provides mcx_error() (src/mcx_utils.c:1314), the engine records its

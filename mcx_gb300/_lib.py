@@ -37,6 +37,8 @@ lib.mcxg_validatecfg.argtypes = [_CFG]
 lib.mcxg_validatecfg.restype = C.c_int
 lib.mcxg_maskdet.argtypes = [_CFG]
 lib.mcxg_maskdet.restype = None
+lib.mcxg_widen_labels.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_uint, C.c_uint, C.c_uint, C.c_void_p]
+lib.mcxg_widen_labels.restype = C.c_int
 lib.mcxg_last_error.argtypes = []
 lib.mcxg_last_error.restype = C.c_char_p
 lib.mcxg_last_error_id.argtypes = []
@@ -115,7 +117,7 @@ lib.mcxg_dn_last_error.restype = C.c_char_p
 
 EXPORTED = [
     "mcx_run_simulation", "mcx_list_gpu", "mcxg_run_simulation_fp64", "mcxg_initcfg", "mcxg_validatecfg",
-    "mcxg_maskdet", "mcxg_last_error", "mcxg_last_error_id", "mcxg_clear_error", "mcxg_set_error", "mcxg_get_stats",
+    "mcxg_maskdet", "mcxg_widen_labels", "mcxg_last_error", "mcxg_last_error_id", "mcxg_clear_error", "mcxg_set_error", "mcxg_get_stats",
     "mcxg_rng_test", "mcxg_photon_stream", "mcxg_session_create", "mcxg_session_reset", "mcxg_session_run",
     "mcxg_session_read", "mcxg_session_destroy", "mcxg_set_launch", "mcxg_run_noalloc", "mcxg_noalloc_scratch_bytes",
     "mcxg_set_seeding", "mcxg_probe_atomic_rate",

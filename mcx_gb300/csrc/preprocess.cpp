@@ -20,6 +20,8 @@
 #include <cstring>
 #include <ctime>
 #include <algorithm>
+#include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -310,6 +312,59 @@ void row_to_column_major(const uint32_t* src, uint32_t* dst, uint3 d) {
     for (auto& t : th) t.join();
 }
 
+// Runs f(begin, end) over [0, n) on up to eight threads, alone below `least` items a thread.
+template <class F>
+void in_parallel(size_t n, size_t least, F&& f) {
+    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t nt = std::min<size_t>({hw, 8, n / std::max<size_t>(1, least)});
+    if (nt < 2) {
+        f((size_t)0, n);
+        return;
+    }
+    std::vector<std::thread> th;
+    th.reserve(nt);
+    size_t t = 0;
+    try {
+        for (; t + 1 < nt; t++) th.emplace_back(f, n * t / nt, n * (t + 1) / nt);
+    } catch (const std::system_error&) {        // no thread to be had: the caller does what is left
+    }
+    f(n * t / nt, n);
+    for (auto& x : th) x.join();
+}
+
+uint32_t max_label(const uint32_t* vol, size_t n) {
+    std::mutex mu;
+    uint32_t most = 0;
+    in_parallel(n, (size_t)1 << 20, [&](size_t a, size_t b) {
+        uint32_t m[8] = {0, 0, 0, 0, 0, 0, 0, 0};       // eight at a time, so that the loop vectorises
+        size_t i = a;
+        for (; i + 8 <= b; i += 8)
+            for (int k = 0; k < 8; k++) m[k] = std::max(m[k], vol[i + k] & kMED_MASK);
+        for (; i < b; i++) m[0] = std::max(m[0], vol[i] & kMED_MASK);
+        std::lock_guard<std::mutex> g(mu);
+        most = std::max(most, *std::max_element(m, m + 8));
+    });
+    return most;
+}
+
+// Labels of any integer type, as C converts them to 32 bits, from [x][y][z] order to MCX's x-fastest
+// order: one pass over a source a quarter of the size of the result, by y rows in 32 x 32 tiles.
+template <class T>
+void widen_labels(const T* src, uint3 d, uint32_t* dst) {
+    constexpr uint32_t E = 32;
+    in_parallel(d.y, std::max<size_t>(1, ((size_t)1 << 18) / std::max<size_t>(1, (size_t)d.x * d.z)), [=](size_t y0, size_t y1) {
+        for (uint32_t x0 = 0; x0 < d.x; x0 += E)
+            for (uint32_t z0 = 0; z0 < d.z; z0 += E)
+                for (size_t y = y0; y < y1; y++) {
+                    const uint32_t x1 = std::min(d.x, x0 + E), z1 = std::min(d.z, z0 + E);
+                    for (uint32_t z = z0; z < z1; z++) {
+                        uint32_t* o = dst + ((size_t)z * d.y + y) * d.x;
+                        for (uint32_t x = x0; x < x1; x++) o[x] = (uint32_t)src[((size_t)x * d.y + y) * d.z + z];
+                    }
+                }
+    });
+}
+
 void validate(Config* cfg) {
     // replay of saved photons (src/mcx_utils.c:1651-1664)
     if (cfg->seed == kSEED_FROM_FILE && (cfg->respin > 1 || cfg->respin < 0)) {
@@ -409,8 +464,7 @@ void validate(Config* cfg) {
     if (cfg->srcpos.w == 0.f) cfg->srcpos.w = 1.f;
     const size_t nvox = (size_t)cfg->dim.x * cfg->dim.y * cfg->dim.z;
     if (cfg->mediabyte <= 4) {
-        uint32_t maxlabel = 0;
-        for (size_t i = 0; i < nvox; i++) maxlabel = std::max(maxlabel, cfg->vol[i] & kMED_MASK);
+        const uint32_t maxlabel = max_label(cfg->vol, nvox);
         if (cfg->medianum <= maxlabel) MCXG_RAISE(-4, "input media optical properties are less than the labels in the volume");
     }
 
@@ -474,6 +528,23 @@ void validate(Config* cfg) {
 // exp(-sum mua_m ppath_m), time of flight sum ppath_m n_m / c0 and detector id.  detps holds
 // dimdetps[1] records of dimdetps[0] floats (savedetflag with D and P); seeds arrive in
 // cfg->replay.seed, seedbyte bytes per photon, and are compacted in place.  Sets nphoton.
+extern "C" int mcxg_widen_labels(const void* src, int itemsize, int is_signed, unsigned nx, unsigned ny, unsigned nz,
+                                 uint32_t* dst) {
+    if (!src || !dst || !nx || !ny || !nz) return -4;
+    const uint3 d{nx, ny, nz};
+    switch (itemsize * (is_signed ? -1 : 1)) {
+        case 1: widen_labels((const uint8_t*)src, d, dst); return 0;
+        case 2: widen_labels((const uint16_t*)src, d, dst); return 0;
+        case 4: widen_labels((const uint32_t*)src, d, dst); return 0;
+        case 8: widen_labels((const uint64_t*)src, d, dst); return 0;
+        case -1: widen_labels((const int8_t*)src, d, dst); return 0;
+        case -2: widen_labels((const int16_t*)src, d, dst); return 0;
+        case -4: widen_labels((const int32_t*)src, d, dst); return 0;
+        case -8: widen_labels((const int64_t*)src, d, dst); return 0;
+        default: return -4;
+    }
+}
+
 extern "C" int mcxg_replayinit(Config* cfg, const float* detps, const int dimdetps[2], int seedbyte) {
     mcxg_clear_error();
     try {

@@ -1605,6 +1605,17 @@ __global__ void merge_kernel(float* __restrict__ out, const float* __restrict__ 
     }
 }
 
+// host += (field + shadow or field64) * scale, the caller's field in host memory, rounded as merge_kernel and
+// a host addition round it.
+__global__ void merge_add_kernel(float* __restrict__ host, const float* __restrict__ field, const float* __restrict__ shadow,
+                                 const double* __restrict__ f64, size_t n, float scale, int positive_only) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        float v = f64 ? (float)f64[i] : field[i] + (shadow ? shadow[i] : 0.f);
+        if (!(positive_only && v < 0.f)) v = __fmul_rn(v, scale);
+        host[i] = __fadd_rn(host[i], v);
+    }
+}
+
 }  // namespace
 
 // The plain path (transport_lean.cuh): what its kernel leaves out must be off.  No photon reaches
@@ -1774,6 +1785,15 @@ cudaError_t launch_merge_field(float* out, const float* field, const float* shad
     const int block = 256;
     const size_t g = (n + block - 1) / block;
     merge_kernel<<<(unsigned)(g < 4096 ? (g ? g : 1) : 4096), block, 0, stream>>>(out, field, shadow, field64, n, scale, positive_only);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_merge_add_field(float* host, const float* field, const float* shadow, const double* field64, size_t n,
+                                   float scale, int positive_only, cudaStream_t stream) {
+    const int block = 256;
+    const size_t g = (n + block - 1) / block;
+    merge_add_kernel<<<(unsigned)(g < 4096 ? (g ? g : 1) : 4096), block, 0, stream>>>(host, field, shadow, field64, n, scale,
+                                                                                     positive_only);
     return cudaGetLastError();
 }
 

@@ -237,5 +237,8 @@ cudaError_t launch_labels_from_vol(const uint32_t* d_vol, uint8_t* d_labels, siz
                                    unsigned int* d_err, cudaStream_t stream);
 cudaError_t launch_merge_field(float* out, const float* field, const float* shadow, const double* field64, size_t n,
                                float scale, int normalize_positive_only, cudaStream_t stream);
+// The same, added to a field in host memory (a device that uses the host's page tables).
+cudaError_t launch_merge_add_field(float* host, const float* field, const float* shadow, const double* field64, size_t n,
+                                   float scale, int normalize_positive_only, cudaStream_t stream);
 
 }  // namespace mcxg
