@@ -407,6 +407,8 @@ struct Session {
     KParams kp{};
     bool reflect = false, savedet = false, use64 = false;
     int block = 256, grid = 0, sms = 0;
+    int run_grid = 0;          // CTAs of the last launch: `grid` or fewer for a run of few photons
+    bool fixed_grid = false;   // CTAs per SM given by mcxg_set_launch
     size_t smem = 0;
     size_t nvox = 0, fieldlen = 0;
     int totalgates = 1;
@@ -742,6 +744,7 @@ struct Session {
         }
         if (bps <= 0) MCXG_RAISE(-6, "the transport kernel does not fit on this device");
         if (o.blocks_per_sm > 0) bps = std::min(bps, o.blocks_per_sm);
+        fixed_grid = o.blocks_per_sm > 0;
         grid = bps * sms;
         kp.chunk = o.chunk > 0 ? o.chunk : 64;
     }
@@ -834,8 +837,9 @@ struct Session {
             kp.mcx_odd = (unsigned)(n - (uint64_t)kp.mcx_per * mcx_streams);
         }
         CK(cudaMemsetAsync(work.p, 0, sizeof(unsigned long long), stream));
+        run_grid = (kp.seed_mode == 1 || fixed_grid) ? grid : transport_grid(kp, grid, block, sms, n);
         CK(cudaEventRecord(ev0, stream));
-        CK(launch_transport(kp, reflect, savedet, grid, block, smem, stream));
+        CK(launch_transport(kp, reflect, savedet, run_grid, block, smem, stream));
         CK(cudaEventRecord(ev1, stream));
         beside();
         CK(cudaEventSynchronize(ev1));
@@ -932,7 +936,7 @@ struct Session {
         st->n_launch = c[kCntLaunch]; st->n_photon = c[kCntPhoton]; st->n_detected = detected();
         st->n_tile_deposit = c[kCntTileDeposit];
         st->kernel_ms = kernel_ms;
-        st->grid = grid; st->block = block; st->chunk = kp.chunk; st->launches = launches;
+        st->grid = run_grid ? run_grid : grid; st->block = block; st->chunk = kp.chunk; st->launches = launches;
         st->error_flags = ef;
     }
 };

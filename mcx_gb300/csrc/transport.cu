@@ -1668,11 +1668,13 @@ static const void* pick_lean(bool reflect, bool savedet) {
     return savedet ? (const void*)lean_kernel<false, true, AREA, M> : (const void*)lean_kernel<false, false, AREA, M>;
 }
 
-// The pencil variants run at 4 CTAs of 256 per SM (64 registers) unless the tuner asks for 3;
-// the variants with the general launch need more registers and run at 3 (80 registers).
+// The general pencil variants run at 4 CTAs of 256 per SM (64 registers) unless the tuner asks for 3; the
+// variants with the general launch need more registers and run at 3 (80 registers), and so do the plain-path
+// ones: at 64 registers they spill nothing but keep fewer constants and addresses (cube, 1e5 photons 2.89 against
+// 2.30 ms, 1e6 4.39 against 3.81, 8e6 17.3 against 16.9; layered head, 1e6, 27.8 against 25.9; 48 registers 37.0).
 static const void* pick(bool reflect, bool savedet, int mode) {
     if (mode == kLeanArea) return pick_lean<true, 3>(reflect, savedet);
-    if (mode == kLeanPencil) return pick_lean<false, 4>(reflect, savedet);
+    if (mode == kLeanPencil) return pick_lean<false, 3>(reflect, savedet);
     if (mode == 4) return pick_flags<3, 4>(reflect, savedet);
     if (mode == 3) return pick_flags<3, 3>(reflect, savedet);
     if (mode == 2) return pick_flags<3, 2>(reflect, savedet);
@@ -1686,6 +1688,20 @@ int transport_blocks_per_sm(bool reflect, bool savedet, int mode, int block, siz
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, block, smem_bytes) != cudaSuccess) return 0;
     return n;
+}
+
+// A run of few photons lasts as long as its longest one, step after step of one warp, and warps beside it on the
+// SM make its steps longer: fewer CTAs, so that a thread has about four photons, end sooner.  Measured (ms, 1 / 2 / 3
+// CTAs an SM): homogeneous cube, 1e5 photons 1.71 / 1.88 / 2.30; 3e5 2.26 / 2.22 / 2.70; 1e6 4.80 / 3.63 / 3.75; layered head
+// 256^3, 1e5 11.9 / 12.6 / 14.2 and 1e6 35.9 / 26.5 / 25.9.
+// Not where a face mirrors photons or hands them to the other side: they all live as long, and the fuller SM wins
+// (cyclic cube, 3e5: 10.6 with 2 CTAs, 8.7 with 3).
+int transport_grid(const KParams& p, int grid, int block, int sms, unsigned long long n) {
+    for (int i = 0; i < 6; i++)
+        if (p.bc[i] == BC_MIRROR || p.bc[i] == BC_CYCLIC) return grid;
+    const unsigned long long a_round = 4ull * (unsigned)block * (unsigned)sms;
+    const unsigned long long rounds = (n + a_round - 1) / a_round;
+    return (unsigned long long)grid <= rounds * (unsigned)sms ? grid : (int)(std::max(rounds, 1ull) * (unsigned)sms);
 }
 
 void place_tile(KParams& k, int kb) {

@@ -211,6 +211,8 @@ int transport_mode(const KParams& p);
 bool transport_general(const KParams& p);
 // Occupancy-derived CTAs per SM for the chosen variant.
 int transport_blocks_per_sm(bool reflect, bool savedet, int mode, int block, size_t smem_bytes);
+// CTAs to launch for n photons on their own streams, at most `grid` (whole CTAs on every one of `sms` SMs).
+int transport_grid(const KParams& p, int grid, int block, int sms, unsigned long long n);
 
 // Source fields of KParams from a preprocessed Config: shape parameters, the pencil's launch
 // state (void skipping traced on the host), the point sources' launch voxel.  d_pattern holds

@@ -49,13 +49,35 @@ inline size_t lean_smem_bytes(const KParams& p, bool savedet) {
     return b;
 }
 
+// transmit() with the roundings the compiler gives it in transport_kernel spelt out: left to itself it fuses the sums of
+// squares one way or the other by what surrounds them, and the photons part.
+__device__ __forceinline__ void transmit_as_general(float& vx, float& vy, float& vz, float n1, float n2, int axis) {
+    const float r = __fdividef(n1, n2);
+    vx = __fmul_rn(vx, r); vy = __fmul_rn(vy, r); vz = __fmul_rn(vz, r);
+    const float a = axis == 0 ? vy : vx, b = axis == 2 ? vy : vz, v = axis == 0 ? vx : (axis == 1 ? vy : vz);
+    const float s = __fmaf_rn(a, a, __fmul_rn(b, b));
+    const float q = (s < 1.f) ? sqrtf(__fsub_rn(1.f, s)) * (float)((v > 0.f) - (v < 0.f)) : 0.f;
+    vx = axis == 0 ? q : vx;
+    vy = axis == 1 ? q : vy;
+    vz = axis == 2 ? q : vz;
+    const float k = rsqrtf(__fmaf_rn(vz, vz, __fmaf_rn(vy, vy, __fmul_rn(vx, vx))));
+    vx = __fmul_rn(vx, k); vy = __fmul_rn(vy, k); vz = __fmul_rn(vz, k);
+}
+
 __device__ __forceinline__ float ahead(float v) { return v > 0.f ? 1.f : 0.f; }
+
+// A warp launches its lanes anew when this many are out of photons.  Sampling an area source and walking its photon
+// through the void is long, and run for one lane it holds 31: four at a time took the planar source from 14.2 to
+// 11.7 ms at 3e6 photons (2: 13.1, 3: 12.0, 6: 11.8, 8: 11.9).  A pencil's launch is short: waiting for a second
+// lane costs what it saves (16.9 -> 17.1 ms on the cube at 8e6).
+template <bool AREA>
+constexpr unsigned kLeanTogether = AREA ? 4u : 1u;
 
 template <bool REFLECT, bool SAVEDET, bool AREA, int MINB>
 __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_constant__ KParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     LeanSmem& S = *reinterpret_cast<LeanSmem*>(smem_raw);
-    constexpr unsigned B = kLeanBlock;
+    constexpr unsigned B = kLeanBlock, kTogether = kLeanTogether<AREA>;
     unsigned* const tile = reinterpret_cast<unsigned*>(S.ppath) + (SAVEDET ? P.partialdata * B : 0u);
     const unsigned tid = threadIdx.x;
     const unsigned lane = tid & 31u;
@@ -80,7 +102,8 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
     }
     __syncthreads();
 
-    bool alive = false;
+    bool alive = false, ended = false;  // ended: its photon has ended and is not accounted for yet
+    unsigned fate = 0u;                 // how, for the detectors: the reference's detector flag
     bool drained = P.src_ok == 0;       // warp-uniform: no photon left to draw
     float px = 0.f, py = 0.f, pz = 0.f, vx = 0.f, vy = 0.f, vz = 1.f, rvx = 0.f, rvy = 0.f, rvz = 0.f;
     float fx = 0.f, fy = 0.f, fz = 0.f; // integer coordinates of the current voxel, as floats
@@ -101,13 +124,42 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
     // the step cap ends a photon 1023 steps past it, the latest transport_kernel does
     const unsigned limit = P.step_cap < 0xFFFFFC00u ? P.step_cap + 1023u : 0xFFFFFFFFu;
 
+    // The end of a photon: detection and energy bookkeeping (src/mcx_core.cu:1113-1182, 365-417)
+    const auto finish = [&]() {
+        ended = false;
+        bool detected = false;
+        if (SAVEDET && (fate & kDET_MASK)) {
+            const int detid = (fate == kOUT_MIN) ? -1 : find_detector(P, px, py, pz);
+            if (detid) {
+                detected = true;
+                const unsigned slot = atomicAdd(P.detcount, 1u);
+                if (slot < P.maxdet) {
+                    float* rec = P.detp + (size_t)slot * P.reclen;
+                    unsigned k = 0;
+                    if (P.savedetflag & 0x1u) rec[k++] = (float)detid;
+                    for (unsigned i = 0; i < P.partialdata; i++) rec[k++] = S.ppath[i * B + tid];
+                    if (P.savedetflag & 0x10u) { rec[k++] = px; rec[k++] = py; rec[k++] = pz; }
+                    if (P.savedetflag & 0x20u) { rec[k++] = vx; rec[k++] = vy; rec[k++] = vz; }
+                    if (P.savedetflag & 0x40u) rec[k++] = S.wlaunch[tid];
+                }
+            }
+        }
+        S.tally[kELaunch * B + tid] += S.wlaunch[tid];
+        S.tally[(detected ? kEDetect : kEEscape) * B + tid] += w;
+        S.tally[kEAbsDep * B + tid] += eabs;
+        S.tally[kEAbsOther * B + tid] += (S.wlaunch[tid] - w) - eabs;
+        S.steps[tid] += limit - left;
+        if (left == 0u) atomicOr(P.errflag, kErrStepCap);
+    };
+
     while (true) {
         // ---- relaunch lanes that have no photon (warp-uniform control flow) ------------------
         const unsigned live = __ballot_sync(kFull, alive);
         if (live != kFull) {
-            if (drained) {
-                if (!live) break;
-            } else {
+            const unsigned idle = __popc(~live);
+            if (!live || (!drained && idle >= kTogether)) {
+                if (AREA && ended) finish();
+                if (drained) break;
                 const unsigned want = ~live;
                 const unsigned cnt = __popc(want);
                 const unsigned rank = __popc(want & ((1u << lane) - 1u));
@@ -373,7 +425,7 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
                     Rtotal = (Rtotal + __fdividef(ctheta - stheta, ctheta + stheta)) * 0.5f;
                 }
                 if (Rtotal < 1.f && !(med == 0u && bcf == BC_MIRROR) && rng_next(r0, r1) > Rtotal) {
-                    transmit(vx, vy, vz, n1, n2, axis);
+                    transmit_as_general(vx, vy, vz, n1, n2, axis);
                     if (med == 0u) {
                         kill = true;
                         detflag = (!valid && P.bc[(outmax ? 9 : 6) + axis]) ? kOUT_MIN : detold;
@@ -429,31 +481,11 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
             rmus = iv.x; rmua = iv.y;
             continue;
         }
-        // terminate: detection and energy bookkeeping (src/mcx_core.cu:1113-1182, 365-417)
-        bool detected = false;
-        if (SAVEDET && (detflag & kDET_MASK) && med == 0u) {
-            const int detid = (detflag == kOUT_MIN) ? -1 : find_detector(P, px, py, pz);
-            if (detid) {
-                detected = true;
-                const unsigned slot = atomicAdd(P.detcount, 1u);
-                if (slot < P.maxdet) {
-                    float* rec = P.detp + (size_t)slot * P.reclen;
-                    unsigned k = 0;
-                    if (P.savedetflag & 0x1u) rec[k++] = (float)detid;
-                    for (unsigned i = 0; i < P.partialdata; i++) rec[k++] = S.ppath[i * B + tid];
-                    if (P.savedetflag & 0x10u) { rec[k++] = px; rec[k++] = py; rec[k++] = pz; }
-                    if (P.savedetflag & 0x20u) { rec[k++] = vx; rec[k++] = vy; rec[k++] = vz; }
-                    if (P.savedetflag & 0x40u) rec[k++] = S.wlaunch[tid];
-                }
-            }
-        }
-        S.tally[kELaunch * B + tid] += S.wlaunch[tid];
-        S.tally[(detected ? kEDetect : kEEscape) * B + tid] += w;
-        S.tally[kEAbsDep * B + tid] += eabs;
-        S.tally[kEAbsOther * B + tid] += (S.wlaunch[tid] - w) - eabs;
-        S.steps[tid] += limit - left;
-        if (left == 0u) atomicOr(P.errflag, kErrStepCap);
+        // the photon ends (an area source's lane keeps its last state until its warp launches some together)
         alive = false;
+        ended = true;
+        fate = (SAVEDET && med == 0u) ? detflag : 0u;
+        if (!AREA) finish();
     }
 
     // ---- flush: tile, tallies, counters ------------------------------------------------------
