@@ -20,10 +20,13 @@
 //   * conditions on the way are evaluated without short cuts and the crossed axis by selection:
 //     branches there ran three versions of the crossing for a few lanes each (13 lanes per
 //     instruction; 44.5 against 37.1 ms on the sphere deck at 8e6 photons).
-// Measured, kernel time before and now (GB300, 2070 MHz): sphere with 50 gates and four detectors,
-// 2e6 photons, 18.4 -> 12.3 ms; layered 128^3 head, 3e5, 43.3 -> 25.8; planar source, 1e6, 9.24 -> 6.07;
-// homogeneous cube, 2e6, 7.99 -> 6.18 and 1e4 photons, 2.86 -> 1.54.  Thread instructions per step on the
-// homogeneous cube 223 -> 179.
+//   * truth values do not outlive a branch: seven predicates do not hold them, and packing and unpacking
+//     them cost 12 of 179 thread instructions a step (17.1 -> 16.5 ms on the cube at 8e6 photons).
+// Measured, kernel time in transport_kernel and here (GB300, 2070 MHz): sphere with 50 gates and four
+// detectors, 2e6 photons, 18.4 -> 11.8 ms; layered 128^3 head, 3e5, 43.3 -> 18.7; planar source, 1e6, 9.24 ->
+// 5.20; homogeneous cube, 2e6, 7.99 -> 5.65 and 1e4 photons, 2.86 -> 1.45.  On the cube 167 thread instructions
+// a step instead of 223, 15.6 lanes an instruction, 82% of the issue slots: what binds it is issue still, the
+// scattering and the crossing block each run by the half of the lanes that need it.
 
 constexpr int kLeanBlock = 256, kLeanWarps = kLeanBlock / 32;
 
@@ -63,6 +66,8 @@ __device__ __forceinline__ void transmit_as_general(float& vx, float& vy, float&
     const float k = rsqrtf(__fmaf_rn(vz, vz, __fmaf_rn(vy, vy, __fmul_rn(vx, vx))));
     vx = __fmul_rn(vx, k); vy = __fmul_rn(vy, k); vz = __fmul_rn(vz, k);
 }
+
+constexpr unsigned kOutside = 0xFFFFFFFFu;      // no voxel's index: a volume has fewer than 2^32 - 1 voxels
 
 __device__ __forceinline__ float ahead(float v) { return v > 0.f ? 1.f : 0.f; }
 
@@ -104,7 +109,9 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
 
     bool alive = false, ended = false;  // ended: its photon has ended and is not accounted for yet
     unsigned fate = 0u;                 // how, for the detectors: the reference's detector flag
-    bool drained = P.src_ok == 0;       // warp-uniform: no photon left to draw
+    // warp-uniform: dead lanes that make the warp draw photons; out of reach when there are none left
+    constexpr unsigned kNever = 64u;
+    unsigned refill_at = P.src_ok == 0 ? kNever : kTogether;
     float px = 0.f, py = 0.f, pz = 0.f, vx = 0.f, vy = 0.f, vz = 1.f, rvx = 0.f, rvy = 0.f, rvz = 0.f;
     float fx = 0.f, fy = 0.f, fz = 0.f; // integer coordinates of the current voxel, as floats
     float w = 0.f, w0 = 0.f, t = 0.f, pscat = 0.f, pathlen = 0.f, segp = 0.f;
@@ -157,9 +164,9 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
         const unsigned live = __ballot_sync(kFull, alive);
         if (live != kFull) {
             const unsigned idle = __popc(~live);
-            if (!live || (!drained && idle >= kTogether)) {
+            if (!live || idle >= refill_at) {
                 if (AREA && ended) finish();
-                if (drained) break;
+                if (refill_at == kNever) break;
                 const unsigned want = ~live;
                 const unsigned cnt = __popc(want);
                 const unsigned rank = __popc(want & ((1u << lane) - 1u));
@@ -175,7 +182,7 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
                     if (rank >= avail) mine = base + (rank - avail);
                     pool_next = base + (cnt - avail);
                     pool_end = base + take;
-                    drained = base >= P.d_nwork;
+                    if (base >= P.d_nwork) refill_at = kNever;
                 } else {
                     pool_next += cnt;
                 }
@@ -266,14 +273,14 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
         t = fmaf(len, n, t);                                            // t += len*n/c0, in grid units
         pathlen += len;
         left--;
-        bool kill = (t > P.d_tw1) | (left == 0u);
 
-        // The face crossed, by selection: a branch per axis would run each of the three for its own lanes.
-        const bool ax = dist == hx, ay = !ax & (dist == hy);
-        bool valid = true, inside = true;
-        unsigned labn = lab, idxn = idx;
+        // What the event below needs of a crossing is kept as numbers it compares again: truth values that live
+        // past a branch are packed into registers and unpacked at every step.
+        unsigned labn = lab, idxn = idx;        // idxn: kOutside where the photon leaves the volume
         float fn = 0.f;
         if (cross) {
+            // The face crossed, by selection: a branch per axis would run each of the three for its own lanes.
+            const bool ax = dist == hx, ay = !ax & (dist == hy);
             // only the crossed axis can leave the volume (2169-2186)
             const float va = ax ? vx : (ay ? vy : vz);
             const float fa = ax ? fx : (ay ? fy : fz);
@@ -282,9 +289,9 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
             const bool up = va > 0.f;
             idxn = up ? idx + stride : idx - stride;
             fn = fa + (up ? 1.f : -1.f);
-            inside = (fn >= 0.f) & (fn < la);
-            valid = inside & (idxn < P.nvox);
+            const bool valid = (fn >= 0.f) & (fn < la) & (idxn < P.nvox);
             labn = (unsigned)__ldg(P.labels + (valid ? idxn : idx));
+            idxn = valid ? idxn : kOutside;
 
             // deposit into the voxel just left, time bin taken at exit (2191-2292)
             const float dw = w0 - w;
@@ -324,7 +331,7 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
             fx = ax ? fn : fx;
             fy = ay ? fn : fy;
             fz = (ax | ay) ? fz : fn;
-        } else if (!kill) {
+        } else if (!((t > P.d_tw1) | (left == 0u))) {
             // ---- scattering event: random numbers in MCX's order (scattering length, azimuth,
             // zenith), one generator step for all three
             float u_len, u_phi, u_th;
@@ -351,7 +358,8 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
             if (SAVEDET) carry = lab;
         }
 
-        if (!kill & valid & (((labn ^ lab) & kLabelMask) == 0u)) {
+        bool kill = (t > P.d_tw1) | (left == 0u);
+        if (!kill & (idxn != kOutside) & (((labn ^ lab) & kLabelMask) == 0u)) {
             // the same medium: nothing else to do
             idx = idxn;
             lab = labn;
@@ -361,7 +369,8 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
         }
 
         // ---- event: another medium, the outside, the end of the window or the step cap ----------
-        const int axis = ax ? 0 : (ay ? 1 : 2);
+        const int axis = (dist == hx) ? 0 : ((dist == hy) ? 1 : 2);
+        const bool valid = idxn != kOutside;
         const unsigned idxold = idx, medold = lab & kLabelMask;
         const unsigned detold = (carry & kLabelDet) ? kDET_MASK : 0u;   // mediaidold's detector bit (2167)
         unsigned med = medold;
@@ -377,7 +386,7 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
             } else {
                 // the voxel index has lost step with the coordinates: never read or write out of
                 // the volume; the photon leaves and the host reports the error
-                if (inside) atomicOr(P.errflag, kErrIndex);
+                if (fn >= 0.f && fn < ((axis == 0) ? P.d_fnx : ((axis == 1) ? P.d_fny : P.d_fnz))) atomicOr(P.errflag, kErrIndex);
                 med = 0u;
                 bcf = P.bc[(outmax ? 3 : 0) + axis];
                 carry = 0u;             // a boundary code, never the detector bit
