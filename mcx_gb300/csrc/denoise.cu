@@ -441,6 +441,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 #include "conv3_roll.cuh"
+#include "conv3_wgrad.cuh"
 
 // ---------------------------------------------------------------------------------------------
 // Weight gradient: dW[co, n] += sum_v dY[v, co] * X[v + off(t), ci], n = t*Cin + ci, over the
@@ -622,6 +623,32 @@ __device__ __forceinline__ void store8(bf16* p, const float (&f)[8]) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
     *reinterpret_cast<uint4*>(p) = u;
+}
+
+// The same for channels in whole 16-byte chunks: a thread keeps one chunk of 8 channels and walks rows a grid apart, the
+// block adds its rows through shared memory, one atomic a channel and block.  Bound by the read of dY: 524288 rows of 16
+// channels (17 MB) took 18.7 us with 2-byte loads, one channel a
+// thread and 128 blocks, and take 6.3.
+__global__ void __launch_bounds__(256) bias_grad8_kernel(const bf16* __restrict__ dy, float* __restrict__ db, long long m, int c) {
+    __shared__ float part[256][9];
+    const int cc = c / 8, rows = 256 / cc;
+    const int ch = threadIdx.x % cc, r0 = threadIdx.x / cc;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (long long v = (long long)blockIdx.x * rows + r0; v < m; v += (long long)gridDim.x * rows) {
+        float f[8];
+        load8(dy + v * c + ch * 8, f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] += f[e];
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) part[threadIdx.x][e] = s[e];
+    __syncthreads();
+    if ((int)threadIdx.x < c) {
+        const int k = threadIdx.x / 8, e = threadIdx.x % 8;
+        float t = 0.f;
+        for (int r = 0; r < rows; ++r) t += part[r * cc + k][e];
+        atomicAdd(db + threadIdx.x, t);
+    }
 }
 
 // 2x2x2 average pooling; (d, h, w) are the fine grid's sizes.  One thread per coarse voxel and
@@ -1106,6 +1133,55 @@ int conv_fwd_dispatch(const bf16* x, const bf16* w, const float* bias, const bf1
     return conv_fwd_launch<128, 16, 64, 4, 1, 3>(x, w, bias, mask, y, g, cin, cout, taps, relu, st);
 }
 
+// Launch of conv3_wgrad_kernel.  Returns 1 where its tiles do not fit (the caller takes the general kernel).  A CTA an
+// SM, shared evenly by the groups: fewer CTAs with longer runs, for fewer additions to dW, were never faster (2 x 64^3
+// 16 to 16: 50 runs 23 us, 24 runs 38; 4 x 8^3 64 to 128: 32 runs 17.4, 16 runs 16.1, 8 runs 20).
+template <int COUT>
+int conv3_wgrad_launch(const bf16* dy, const bf16* x, float* dw, Geo g, int cin, cudaStream_t st) {
+    using S = WgradShape<COUT>;
+    auto encode = tensor_map_encoder();
+    if (!encode) return fail("wgrad: cuTensorMapEncodeTiled is not available");
+    const int tx = (g.w + 7) / 8, ty = (g.h + 15) / 16, tz = (g.d + S::PZ - 1) / S::PZ;
+    const long long tiles = (long long)g.nvol * tx * ty * tz;
+    const int pairs = 9 * (cin / 16), groups = (pairs + S::G - 1) / S::G;
+    int nsl = 1;
+    for (int p = 0; p < pairs; p += S::G) {
+        const int n = ((p + S::G < pairs ? p + S::G : pairs) - 1) / 9 - p / 9 + 1;
+        nsl = n > nsl ? n : nsl;
+    }
+    const int stage = S::YBYTES + nsl * S::XSTRIDE;
+    int stages = kRollSmem / stage;
+    if (stages > S::MAX_STAGES) stages = S::MAX_STAGES;
+    if (stages < 2 || tiles >= (1LL << 31)) return 1;
+    CUtensorMap maps[2];
+    for (int m = 0; m < 2; ++m) {
+        // dY [nvol][d][h][w][cout] in boxes of PZ planes of 16 x 8 voxels, X [..][cin] with one voxel more on every side
+        const cuuint64_t c = m ? cin : COUT;
+        const cuuint64_t dims[5] = {c, (cuuint64_t)g.w, (cuuint64_t)g.h, (cuuint64_t)g.d, (cuuint64_t)g.nvol};
+        const cuuint64_t strides[4] = {c * 2, (cuuint64_t)g.w * c * 2, (cuuint64_t)g.h * g.w * c * 2,
+                                       (cuuint64_t)g.d * g.h * g.w * c * 2};
+        const cuuint32_t box[5] = {16, m ? 10u : 8u, m ? 18u : 16u, (cuuint32_t)(m ? S::PZ + 2 : S::PZ), 1};
+        const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+        if (encode(&maps[m], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16*>(m ? x : dy), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return fail("wgrad: cuTensorMapEncodeTiled rejected the layout");
+    }
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int parts = sms / groups;
+    if (parts < 1) parts = 1;
+    if (parts > tiles) parts = (int)tiles;
+    int smem = stages * stage;
+    if (smem < 120 * 1024) smem = 120 * 1024;       // one CTA an SM: each takes all of its tensor memory
+    auto kern = conv3_wgrad_kernel<COUT>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    kern<<<groups * parts, 192, smem, st>>>(maps[0], maps[1], dw, g, cin, tx, ty, tz, (int)tiles, parts, stages,
+                                            (reinterpret_cast<uintptr_t>(dw) & 15u) == 0 ? 1 : 0);
+    return launched();
+}
+
 template <int BM>
 int wgrad_launch(const bf16* dy, const bf16* x, float* dw, Geo g, int cin, int taps, cudaStream_t st) {
     constexpr int STAGES = 4;
@@ -1191,6 +1267,21 @@ int mcxg_dn_conv_wgrad(const void* dy, const void* x, float* dw, int nvol, int d
     auto st = static_cast<cudaStream_t>(stream);
     auto DY = static_cast<const bf16*>(dy);
     auto X = static_cast<const bf16*>(x);
+    // The tensor-memory kernel from 2^19 (voxels x input channels) on.  Either side, the general kernel's time against
+    // it, device us: 8192 voxels 16 to 16 5.9 / 7.6, 8192 32 to 32 7.9 / 8.8, 2048 128 to 128 13.9 / 18.3; 13547 48 to 16
+    // 11.6 / 9.2, 32768 16 to 16 10.3 / 7.7, 16384 64 to 64 22.8 / 13.8, 8192 128 to 128 33.7 / 22.5.  Below it one
+    // CTA's fixed costs (its tensor memory, the walk over its accumulators) are the whole time.
+    if (taps == 27 && use_tcgen05() && (long long)nvol * d * h * wd * cin >= (1 << 19)) {
+        int rc = 1;
+        switch (cout) {
+            case 16: rc = conv3_wgrad_launch<16>(DY, X, dw, g, cin, st); break;
+            case 32: rc = conv3_wgrad_launch<32>(DY, X, dw, g, cin, st); break;
+            case 64: rc = conv3_wgrad_launch<64>(DY, X, dw, g, cin, st); break;
+            case 128: rc = conv3_wgrad_launch<128>(DY, X, dw, g, cin, st); break;
+            default: break;
+        }
+        if (rc != 1) return rc;
+    }
     switch (cout) {
         case 16: return wgrad_launch<16>(DY, X, dw, g, cin, taps, st);
         case 32: return wgrad_launch<32>(DY, X, dw, g, cin, taps, st);
@@ -1203,6 +1294,13 @@ int mcxg_dn_conv_wgrad(const void* dy, const void* x, float* dw, int nvol, int d
 int mcxg_dn_bias_grad(const void* dy, float* db, long long m, int c, void* stream) {
     if (!dy || !db || m <= 0) return fail("bias grad: null tensor or no voxels");
     if (c <= 0 || 256 % c) return fail("bias grad: channels must divide 256");
+    if (c % 8 == 0 && aligned16(dy)) {
+        // about eight rows a thread, at most four blocks an SM
+        const long long rows = 256 / (c / 8), want = (m + 8 * rows - 1) / (8 * rows);
+        bias_grad8_kernel<<<(unsigned)(want < 608 ? want : 608), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+            static_cast<const bf16*>(dy), db, m, c);
+        return launched();
+    }
     long long rows = 4096;
     unsigned blocks = (unsigned)((m + rows - 1) / rows);
     bias_grad_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const bf16*>(dy), db, m, c, rows);
