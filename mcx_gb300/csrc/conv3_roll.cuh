@@ -120,6 +120,14 @@ __device__ __forceinline__ void tma_4d(uint32_t lead, uint32_t dst, const CUtens
         "l"(map), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar), "r"(lead)
         : "memory");
 }
+__device__ __forceinline__ void tma_3d(uint32_t lead, uint32_t dst, const CUtensorMap* map, int a, int b, int c, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %6, 0;\n\t"
+        "@e cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+        "[%5];\n\t}\n" ::"r"(dst),
+        "l"(map), "r"(a), "r"(b), "r"(c), "r"(bar), "r"(lead)
+        : "memory");
+}
 __device__ __forceinline__ void expect_tx(uint32_t lead, uint32_t bar, uint32_t bytes) {
     asm volatile(
         "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t"

@@ -441,6 +441,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 #include "conv3_roll.cuh"
+#include "conv3_stream.cuh"
 #include "conv3_wgrad.cuh"
 
 // ---------------------------------------------------------------------------------------------
@@ -1212,6 +1213,52 @@ int conv3_roll_dispatch(const bf16* x, const bf16* w, const float* bias, const b
 #undef ROLL
 }
 
+// Launch of conv3_stream_kernel.  Returns 1 where two halo planes and two weight buffers don't fit (more than 288 input
+// channels).  Every size it takes is the faster on it, from one voxel (82 -> 23 us at 192 to 64).
+int conv3_stream_launch(const bf16* x, const bf16* w, const float* bias, const bf16* mask, bf16* y, Geo g, int cin,
+                        int cout, int relu, cudaStream_t st) {
+    using S = StreamShape;
+    const int planes = 2 * (cin / 16) * S::ENTRY;
+    int wbufs = (kRollSmem - planes) / S::WCHUNK;
+    if (planes > kRollSmem || wbufs < 2) return 1;
+    if (wbufs > S::MAX_W) wbufs = S::MAX_W;
+    const int tx = (g.w + 7) / 8, ty = (g.h + 15) / 16;
+    const long long tiles = (long long)(cout / S::BN) * g.nvol * g.d * ty * tx;
+    if (tiles >= (1LL << 30)) return 1;
+    auto encode = tensor_map_encoder();
+    if (!encode) return fail("conv: cuTensorMapEncodeTiled is not available");
+    CUtensorMap xmap, wmap;
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    {
+        const cuuint64_t dims[5] = {(cuuint64_t)cin, (cuuint64_t)g.w, (cuuint64_t)g.h, (cuuint64_t)g.d, (cuuint64_t)g.nvol};
+        const cuuint64_t strides[4] = {(cuuint64_t)cin * 2, (cuuint64_t)g.w * cin * 2, (cuuint64_t)g.h * g.w * cin * 2,
+                                       (cuuint64_t)g.d * g.h * g.w * cin * 2};
+        const cuuint32_t box[5] = {16, (cuuint32_t)S::HX, 18, 1, 1};
+        if (encode(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16*>(x), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return fail("conv: cuTensorMapEncodeTiled rejected the activation layout");
+    }
+    {
+        // weights [cout][27][cin]: a box of 64 channels of a tap, rows of output channels
+        const cuuint64_t dims[3] = {(cuuint64_t)cin, 27, (cuuint64_t)cout};
+        const cuuint64_t strides[2] = {(cuuint64_t)cin * 2, (cuuint64_t)27 * cin * 2};
+        const cuuint32_t box[3] = {64, 1, (cuuint32_t)S::BN};
+        if (encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(w), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return fail("conv: cuTensorMapEncodeTiled rejected the weight layout");
+    }
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int smem = wbufs * S::WCHUNK + planes;
+    cudaFuncSetAttribute(conv3_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    conv3_stream_kernel<<<(unsigned)(tiles < sms ? tiles : sms), 224, smem, st>>>(
+        xmap, wmap, bias, mask, y, g, cin, cout, relu, tx, ty, (int)tiles, wbufs, (reinterpret_cast<uintptr_t>(y) & 31u) == 0 ? 1 : 0);
+    return launched();
+}
+
 // Narrow 3x3x3 layers run on tcgen05 unless MCXG_DN_MMA_SYNC=1 selects the warp-level mma.sync
 // halo kernel (kept as the measured baseline of the tensor-core port).
 bool use_tcgen05() {
@@ -1229,7 +1276,8 @@ int conv_fwd_dispatch(const bf16* x, const bf16* w, const float* bias, const bf1
         // 16, 32, 48, 80, 96 .. outputs sum slice by slice, the wider layers tap by tap: the orders of the kernels
         // this one stands in for, kept because a whole network's bf16 roundings follow from them
         const bool narrow = cout % 32 != 0 || (cout / 32 <= 3 && cout % 64 != 0);
-        const int rc = conv3_roll_dispatch(x, w, bias, mask, y, g, cin, cout, relu, !narrow, st);
+        int rc = conv3_roll_dispatch(x, w, bias, mask, y, g, cin, cout, relu, !narrow, st);
+        if (rc == 1 && !narrow && cout % 64 == 0) rc = conv3_stream_launch(x, w, bias, mask, y, g, cin, cout, relu, st);
         if (rc != 1) return rc;
     }
     // narrow 3x3x3 layers: halo tiles (each input voxel loaded once per tile, not once per tap)
