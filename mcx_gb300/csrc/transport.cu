@@ -1649,9 +1649,12 @@ bool transport_general(const KParams& p) { return transport_mode(p) != 0; }
 int transport_mode(const KParams& p) {
     if (p.mediaformat == kMedia2LabelSplit) return 4;
     if (media_words(p.mediaformat)) return 3;
-    if (p.replay || p.saveseed || p.outputtype > kOutEnergy || p.traj || p.polarized || p.saveref || p.srcnum > 1 ||
-        p.nphase > 2 || p.nangle > 0 || p.nextra > 0)
-        return 2;
+    if (p.saveseed || p.traj || p.polarized || p.saveref || p.srcnum > 1 || p.nphase > 2 || p.nangle > 0 || p.nextra > 0) return 2;
+    // (the replay outputs at scattering events, and the complex one, need the general kernel's state; sampled sources
+    // and a replay into flux run there too)
+    if (p.replay && (p.outputtype == kOutJacobian || p.outputtype == kOutWLTOF) && p.srctype == kSrcPencil && lean_path(p))
+        return kLeanReplay;
+    if (p.replay || p.outputtype > kOutEnergy) return 2;
     const int area = (p.srctype != kSrcPencil) ? 1 : 0;
     return lean_path(p) ? kLeanPencil + area : area;
 }
@@ -1662,10 +1665,10 @@ static const void* pick_flags(bool reflect, bool savedet) {
     return savedet ? kernel_ptr<false, true, M, K>() : kernel_ptr<false, false, M, K>();
 }
 
-template <bool AREA, int M>
+template <bool AREA, bool REPLAY, int M>
 static const void* pick_lean(bool reflect, bool savedet) {
-    if (reflect) return savedet ? (const void*)lean_kernel<true, true, AREA, M> : (const void*)lean_kernel<true, false, AREA, M>;
-    return savedet ? (const void*)lean_kernel<false, true, AREA, M> : (const void*)lean_kernel<false, false, AREA, M>;
+    if (reflect) return savedet ? (const void*)lean_kernel<true, true, AREA, REPLAY, M> : (const void*)lean_kernel<true, false, AREA, REPLAY, M>;
+    return savedet ? (const void*)lean_kernel<false, true, AREA, REPLAY, M> : (const void*)lean_kernel<false, false, AREA, REPLAY, M>;
 }
 
 // The general pencil variants run at 4 CTAs of 256 per SM (64 registers) unless the tuner asks for 3; the
@@ -1673,8 +1676,9 @@ static const void* pick_lean(bool reflect, bool savedet) {
 // ones: at 64 registers they spill nothing but keep fewer constants and addresses (cube, 1e5 photons 2.89 against
 // 2.30 ms, 1e6 4.39 against 3.81, 8e6 17.3 against 16.9; layered head, 1e6, 27.8 against 25.9; 48 registers 37.0).
 static const void* pick(bool reflect, bool savedet, int mode) {
-    if (mode == kLeanArea) return pick_lean<true, 3>(reflect, savedet);
-    if (mode == kLeanPencil) return pick_lean<false, 3>(reflect, savedet);
+    if (mode == kLeanReplay) return pick_lean<false, true, 3>(reflect, savedet);
+    if (mode == kLeanArea) return pick_lean<true, false, 3>(reflect, savedet);
+    if (mode == kLeanPencil) return pick_lean<false, false, 3>(reflect, savedet);
     if (mode == 4) return pick_flags<3, 4>(reflect, savedet);
     if (mode == 3) return pick_flags<3, 3>(reflect, savedet);
     if (mode == 2) return pick_flags<3, 2>(reflect, savedet);

@@ -205,8 +205,8 @@ size_t transport_smem_bytes(const KParams& p, int block, bool savedet);
 // Kernel variant of a parameter set: 0 = pencil beam with flux/fluence/energy output, 1 = other
 // source shapes sampled per photon, 2 = replay, seed saving or the replay / path-length outputs,
 // 3 = everything of 2 on a per-voxel media format, 4 = split voxels; kLeanPencil / kLeanArea = 0 / 1
-// on the plain path (transport_lean.cuh).
-constexpr int kLeanPencil = 8, kLeanArea = 9;
+// on the plain path (transport_lean.cuh), kLeanReplay = its replay into the absorption Jacobians.
+constexpr int kLeanPencil = 8, kLeanArea = 9, kLeanReplay = 10;
 int transport_mode(const KParams& p);
 bool transport_general(const KParams& p);
 // Occupancy-derived CTAs per SM for the chosen variant.

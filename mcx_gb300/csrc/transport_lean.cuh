@@ -27,6 +27,11 @@
 // 5.20; homogeneous cube, 2e6, 7.99 -> 5.65 and 1e4 photons, 2.86 -> 1.45.  On the cube 167 thread instructions
 // a step instead of 223, 15.6 lanes an instruction, 82% of the issue slots: what binds it is issue still, the
 // scattering and the crossing block each run by the half of the lanes that need it.
+//
+// REPLAY runs detected photons again from their saved states into the Jacobian of absorption (or its time-of-flight
+// weighted form).  A replay has about a photon a thread, so it lasts as long as its longest photon, and that as its steps:
+// 44 829 photons of the reflecting cube took 5.5 ms in transport_kernel's variant with every replay option and 1.46
+// here; with two media, a void pocket and reflection 6.0 and 1.65.
 
 constexpr int kLeanBlock = 256, kLeanWarps = kLeanBlock / 32;
 
@@ -78,7 +83,7 @@ __device__ __forceinline__ float ahead(float v) { return v > 0.f ? 1.f : 0.f; }
 template <bool AREA>
 constexpr unsigned kLeanTogether = AREA ? 4u : 1u;
 
-template <bool REFLECT, bool SAVEDET, bool AREA, int MINB>
+template <bool REFLECT, bool SAVEDET, bool AREA, bool REPLAY, int MINB>
 __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_constant__ KParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     LeanSmem& S = *reinterpret_cast<LeanSmem*>(smem_raw);
@@ -126,6 +131,8 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
     unsigned long long r0 = 0ull, r1 = 0ull;
     float eabs = 0.f;                   // absorbed weight of the photon recorded in the field
     unsigned left = 0u;                 // steps the photon may still take
+    float rw = 0.f, rtof = 1.f;         // replay: detected weight, time of flight where the output carries it
+    int rbin = -1;                      // replay: its field block (gate + detector offset), -1 none
     unsigned c_scat = 0u, c_dep = 0u, c_tile = 0u;
     S.steps[tid] = 0u;
     // the step cap ends a photon 1023 steps past it, the latest transport_kernel does
@@ -195,7 +202,22 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
                 const bool start = !alive && mine < P.d_nwork;
                 bool entered = false;
                 if (start) {
-                    seed_photon(P.seed, P.photon_offset + mine, r0, r1);
+                    if constexpr (REPLAY) {
+                        // a detected photon again: its saved launch state and detection record
+                        // (src/mcx_core.cu:1203-1211)
+                        r0 = __ldg(P.replay_seed + 2 * mine);
+                        r1 = __ldg(P.replay_seed + 2 * mine + 1);
+                        const float tof = __ldg(P.replay_tof + mine);
+                        rbin = (int)floorf((tof - P.twin0) * P.Rtstep);
+                        if (rbin < 0 || rbin >= P.maxgate) rbin = -1;      // detected outside this gate group
+                        else if (P.replaydet == -1) rbin += ((__ldg(P.replay_detid + mine) & 0xFFFF) - 1) * P.maxgate;
+                        rw = __ldg(P.replay_w + mine);
+                        if (P.outputtype == kOutWLTOF) rtof = tof;
+                        // the draw by which the recorded run picked its source (src/mcx_core.cu:1229-1231)
+                        if (P.srcid >= 1) (void)rng_next(r0, r1);
+                    } else {
+                        seed_photon(P.seed, P.photon_offset + mine, r0, r1);
+                    }
                     if (!AREA || P.srctype == kSrcPencil) {
                         // the pencil's launch state, traced through the void by the host
                         px = P.src_p.x; py = P.src_p.y; pz = P.src_p.z; w = P.src_p.w;
@@ -296,18 +318,20 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
             // deposit into the voxel just left, time bin taken at exit (2191-2292)
             const float dw = w0 - w;
             float weight = (rmua < 0.f) ? (w0 * pathlen) : dw * rmua;
+            if (REPLAY) weight = (rbin < 0) ? 0.f : rw * pathlen * rtof;        // mua Jacobian (x time of flight)
             const bool rec = (t >= P.d_tw0) & (t < P.d_tw1) & (weight != 0.f);
             eabs += rec ? dw : 0.f;
             c_dep += rec;
             // (a deposit that passed the window test may compute bin -1 at a window that does not
             // start at 0: it belongs to the first gate)
             int tshift = 0;
-            if (P.maxgate > 1) tshift = min(P.maxgate - 1, max(0, (int)floorf(fmaf(t, P.d_bin_a, -P.d_bin_b))));
+            if (REPLAY) tshift = rbin;
+            else if (P.maxgate > 1) tshift = min(P.maxgate - 1, max(0, (int)floorf(fmaf(t, P.d_bin_a, -P.d_bin_b))));
             float* const slot = P.field + ((size_t)tshift * P.nvox + idx);
             // the index range of the tile box (empty without a tile) screens most deposits out
             // with one compare before the box test
             bool in_tile = false;
-            if (idx - P.d_tile_lo < P.d_tile_span) {
+            if (!REPLAY && idx - P.d_tile_lo < P.d_tile_span) {
                 const float ox = fx - P.d_tx0, oy = fy - P.d_ty0, oz = fz - P.d_tz0;
                 in_tile = (ox >= 0.f) & (ox < P.d_tnx) & (oy >= 0.f) & (oy < P.d_tny) & (oz >= 0.f) & (oz < P.d_tnz) &
                           rec & (weight > 0.f) & ((unsigned)(tshift - P.tg0) < (unsigned)P.tng);
