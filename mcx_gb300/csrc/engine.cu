@@ -838,6 +838,7 @@ struct Session {
         }
         CK(cudaMemsetAsync(work.p, 0, sizeof(unsigned long long), stream));
         run_grid = (kp.seed_mode == 1 || fixed_grid) ? grid : transport_grid(kp, grid, block, sms, n);
+        kp.spare = transport_spare(run_grid, block, n);
         CK(cudaEventRecord(ev0, stream));
         CK(launch_transport(kp, reflect, savedet, run_grid, block, smem, stream));
         CK(cudaEventRecord(ev1, stream));
@@ -865,6 +866,7 @@ struct Session {
             kp.mcx_per = (unsigned)(n / mcx_streams);
             kp.mcx_odd = (unsigned)(n - (uint64_t)kp.mcx_per * mcx_streams);
         }
+        kp.spare = 0;
         if (fresh) {
             CK(cudaMemsetAsync(field.p, 0, field.bytes, s));
             if (shadow.p) CK(cudaMemsetAsync(shadow.p, 0, shadow.bytes, s));

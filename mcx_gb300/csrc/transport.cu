@@ -1665,20 +1665,22 @@ static const void* pick_flags(bool reflect, bool savedet) {
     return savedet ? kernel_ptr<false, true, M, K>() : kernel_ptr<false, false, M, K>();
 }
 
-template <bool AREA, bool REPLAY, int M>
+template <bool AREA, int KIND, int M>
 static const void* pick_lean(bool reflect, bool savedet) {
-    if (reflect) return savedet ? (const void*)lean_kernel<true, true, AREA, REPLAY, M> : (const void*)lean_kernel<true, false, AREA, REPLAY, M>;
-    return savedet ? (const void*)lean_kernel<false, true, AREA, REPLAY, M> : (const void*)lean_kernel<false, false, AREA, REPLAY, M>;
+    if (reflect) return savedet ? (const void*)lean_kernel<true, true, AREA, KIND, M> : (const void*)lean_kernel<true, false, AREA, KIND, M>;
+    return savedet ? (const void*)lean_kernel<false, true, AREA, KIND, M> : (const void*)lean_kernel<false, false, AREA, KIND, M>;
 }
 
 // The general pencil variants run at 4 CTAs of 256 per SM (64 registers) unless the tuner asks for 3; the
 // variants with the general launch need more registers and run at 3 (80 registers), and so do the plain-path
 // ones: at 64 registers they spill nothing but keep fewer constants and addresses (cube, 1e5 photons 2.89 against
 // 2.30 ms, 1e6 4.39 against 3.81, 8e6 17.3 against 16.9; layered head, 1e6, 27.8 against 25.9; 48 registers 37.0).
-static const void* pick(bool reflect, bool savedet, int mode) {
-    if (mode == kLeanReplay) return pick_lean<false, true, 3>(reflect, savedet);
-    if (mode == kLeanArea) return pick_lean<true, false, 3>(reflect, savedet);
-    if (mode == kLeanPencil) return pick_lean<false, false, 3>(reflect, savedet);
+static const void* pick(bool reflect, bool savedet, int mode, bool few = false) {
+    if (mode == kLeanReplay) return pick_lean<false, kLeanReplays, 3>(reflect, savedet);
+    if (mode == kLeanArea)
+        return few ? pick_lean<true, kLeanFew, 3>(reflect, savedet) : pick_lean<true, kLeanMany, 3>(reflect, savedet);
+    if (mode == kLeanPencil)
+        return few ? pick_lean<false, kLeanFew, 3>(reflect, savedet) : pick_lean<false, kLeanMany, 3>(reflect, savedet);
     if (mode == 4) return pick_flags<3, 4>(reflect, savedet);
     if (mode == 3) return pick_flags<3, 3>(reflect, savedet);
     if (mode == 2) return pick_flags<3, 2>(reflect, savedet);
@@ -1700,12 +1702,24 @@ int transport_blocks_per_sm(bool reflect, bool savedet, int mode, int block, siz
 // 256^3, 1e5 11.9 / 12.6 / 14.2 and 1e6 35.9 / 26.5 / 25.9.
 // Not where a face mirrors photons or hands them to the other side: they all live as long, and the fuller SM wins
 // (cyclic cube, 3e5: 10.6 with 2 CTAs, 8.7 with 3).
+// Where even that leaves every warp of the full grid no more than four photons, the full grid: 1e4 photons, a warp's
+// spread over its lanes as below, 1.35 / 1.30 / 1.23 on the cube, 1.54 / 1.51 / 1.49 with detectors (3e4: 1.49 / 1.53 / 1.68).
 int transport_grid(const KParams& p, int grid, int block, int sms, unsigned long long n) {
     for (int i = 0; i < 6; i++)
         if (p.bc[i] == BC_MIRROR || p.bc[i] == BC_CYCLIC) return grid;
+    if (transport_mode(p) >= kLeanPencil && n <= 4ull * (unsigned)grid * (unsigned)(block / 32)) return grid;
     const unsigned long long a_round = 4ull * (unsigned)block * (unsigned)sms;
     const unsigned long long rounds = (n + a_round - 1) / a_round;
     return (unsigned long long)grid <= rounds * (unsigned)sms ? grid : (int)(std::max(rounds, 1ull) * (unsigned)sms);
+}
+
+// Fewer photons than the plain path's kernel has lanes go to as few lanes of every warp as hold them: a warp's step is
+// shorter the fewer paths its lanes take.  Filling warp after warp left most of them idle: cube, 1e2 photons 1.31 -> 0.85
+// ms, 1e4 1.46 -> 1.35 (with detectors 1.75 -> 1.54); layered head 256^3, 1e4, 10.6 -> 8.9.  Not where other launches share
+// the SMs, which a full warp loads less.
+unsigned transport_spare(int grid, int block, unsigned long long n) {
+    const unsigned long long warps = (unsigned long long)grid * (unsigned)(block / 32), per = (n + warps - 1) / warps;
+    return per < 32ull ? 32u - (unsigned)std::max(per, 1ull) : 0u;
 }
 
 void place_tile(KParams& k, int kb) {
@@ -1770,7 +1784,7 @@ cudaError_t launch_transport(const KParams& in, bool reflect, bool savedet, int 
     if (p.d_nwork < (unsigned long long)grid * (unsigned long long)block * 16ull) p.chunk = 1;
     // the caller sized the shared memory for the variant of its parameters: never launch another's
     if (smem_bytes < transport_smem_bytes(p, block, savedet)) return cudaErrorInvalidValue;
-    const void* k = pick(reflect, savedet, transport_mode(p));
+    const void* k = pick(reflect, savedet, transport_mode(p), p.spare > 0u);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
     if (e != cudaSuccess) return e;
     void* args[] = {const_cast<KParams*>(&p)};

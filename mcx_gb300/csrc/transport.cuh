@@ -152,6 +152,7 @@ struct KParams {
     unsigned long long seed;
     unsigned long long* work;       // photon counter the persistent warps draw chunks from
     int chunk;                      // photons per warp refill
+    unsigned spare;                 // plain path: lanes of a warp left without a photon
     unsigned int step_cap;          // safety cap on steps per photon (error flag when hit)
 
     // --- RNG seeding: 0 = one stream per photon from (seed, photon index); 1 = MCX's scheme, one
@@ -213,6 +214,8 @@ bool transport_general(const KParams& p);
 int transport_blocks_per_sm(bool reflect, bool savedet, int mode, int block, size_t smem_bytes);
 // CTAs to launch for n photons on their own streams, at most `grid` (whole CTAs on every one of `sms` SMs).
 int transport_grid(const KParams& p, int grid, int block, int sms, unsigned long long n);
+// Lanes of a warp left without a photon in a run of n (KParams::spare), for a launch that has the GPU to itself.
+unsigned transport_spare(int grid, int block, unsigned long long n);
 
 // Source fields of KParams from a preprocessed Config: shape parameters, the pencil's launch
 // state (void skipping traced on the host), the point sources' launch voxel.  d_pattern holds

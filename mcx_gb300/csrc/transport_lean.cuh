@@ -83,11 +83,17 @@ __device__ __forceinline__ float ahead(float v) { return v > 0.f ? 1.f : 0.f; }
 template <bool AREA>
 constexpr unsigned kLeanTogether = AREA ? 4u : 1u;
 
-template <bool REFLECT, bool SAVEDET, bool AREA, bool REPLAY, int MINB>
+// What a launch of the kernel is for: photons by the thousand a warp; few of them, spread over all warps (in the same kernel
+// the spare lanes' arithmetic cost the long runs 1%); a replay.
+enum LeanKind : int { kLeanMany = 0, kLeanFew, kLeanReplays };
+
+template <bool REFLECT, bool SAVEDET, bool AREA, int KIND, int MINB>
 __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_constant__ KParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     LeanSmem& S = *reinterpret_cast<LeanSmem*>(smem_raw);
     constexpr unsigned B = kLeanBlock, kTogether = kLeanTogether<AREA>;
+    constexpr bool REPLAY = KIND == kLeanReplays;
+    const unsigned spare = KIND == kLeanMany ? 0u : P.spare;        // lanes left without a photon
     unsigned* const tile = reinterpret_cast<unsigned*>(S.ppath) + (SAVEDET ? P.partialdata * B : 0u);
     const unsigned tid = threadIdx.x;
     const unsigned lane = tid & 31u;
@@ -116,7 +122,7 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
     unsigned fate = 0u;                 // how, for the detectors: the reference's detector flag
     // warp-uniform: dead lanes that make the warp draw photons; out of reach when there are none left
     constexpr unsigned kNever = 64u;
-    unsigned refill_at = P.src_ok == 0 ? kNever : kTogether;
+    unsigned refill_at = P.src_ok == 0 ? kNever : kTogether + spare;
     float px = 0.f, py = 0.f, pz = 0.f, vx = 0.f, vy = 0.f, vz = 1.f, rvx = 0.f, rvy = 0.f, rvz = 0.f;
     float fx = 0.f, fy = 0.f, fz = 0.f; // integer coordinates of the current voxel, as floats
     float w = 0.f, w0 = 0.f, t = 0.f, pscat = 0.f, pathlen = 0.f, segp = 0.f;
@@ -175,7 +181,7 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
                 if (AREA && ended) finish();
                 if (refill_at == kNever) break;
                 const unsigned want = ~live;
-                const unsigned cnt = __popc(want);
+                const unsigned cnt = idle - spare;
                 const unsigned rank = __popc(want & ((1u << lane) - 1u));
                 unsigned long long pool_next = S.pool[2 * warp], pool_end = S.pool[2 * warp + 1];
                 const unsigned long long avail = pool_end - pool_next;
@@ -199,7 +205,7 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
                     S.pool[2 * warp + 1] = pool_end;
                 }
                 __syncwarp();               // and reads the new one at the next refill
-                const bool start = !alive && mine < P.d_nwork;
+                const bool start = !alive && mine < P.d_nwork && (KIND == kLeanMany || rank < cnt);
                 bool entered = false;
                 if (start) {
                     if constexpr (REPLAY) {
