@@ -213,6 +213,7 @@ __global__ void __launch_bounds__(320, 1) conv3_roll_kernel(const __grid_constan
     __shared__ __align__(8) uint64_t s_bar[2 * S::MAX_STAGES + 2 * S::MAX_W + 2 * RP];
     __shared__ uint32_t s_tmem;
 
+    chain_next();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int slices = cin / 16;
     const bool resident = wbufs >= slices;
@@ -246,6 +247,7 @@ __global__ void __launch_bounds__(320, 1) conv3_roll_kernel(const __grid_constan
 
     bool fault = false;
     RollRun run(planes, g, tiles_y, tiles_x, chunk, BN);
+    chain_wait();
     if (TAPS && warp == 8) {
         // ---- TMA copies, tap-major: every slice's weights, then halo planes slice by slice ------------
         const uint32_t lead = elect_lead();

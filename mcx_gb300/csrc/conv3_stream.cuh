@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(224, 1) conv3_stream_kernel(const __grid_const
     __shared__ __align__(8) uint64_t s_bar[2 * S::MAX_W + 8];
     __shared__ uint32_t s_tmem;
 
+    chain_next();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int slices = cin / 16, chunks = (cin + 63) / 64;
     const uint32_t sw = smem_addr(dyn_smem), sh = sw + wbufs * S::WCHUNK, plane = slices * S::ENTRY;
@@ -85,6 +86,7 @@ __global__ void __launch_bounds__(224, 1) conv3_stream_kernel(const __grid_const
 
     bool fault = false;
     StreamTile tile(tiles, tiles_x, tiles_y, g);
+    chain_wait();
     if (warp == 4) {
         const uint32_t lead = elect_lead();
         RollRing st(2);

@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(192, 1) conv3_wgrad_kernel(const __grid_consta
     __shared__ __align__(8) uint64_t s_bar[2 * S::MAX_STAGES + 1];
     __shared__ uint32_t s_tmem;
 
+    chain_next();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int group = (int)blockIdx.x / parts, part = (int)blockIdx.x % parts;
     const int pair0 = group * S::G, pairs = min(S::G, 9 * (cin / 16) - pair0);    // pair = slice * 9 + dydx
@@ -60,8 +61,6 @@ __global__ void __launch_bounds__(192, 1) conv3_wgrad_kernel(const __grid_consta
     const int t_lo = (int)((long long)tiles * part / parts), t_hi = (int)((long long)tiles * (part + 1) / parts);
     const uint32_t sh = smem_addr(dyn_smem), stage_bytes = S::YBYTES + nsl * S::XSTRIDE;
     const uint32_t full0 = smem_addr(s_bar), empty0 = full0 + 8 * S::MAX_STAGES, done = empty0 + 8 * S::MAX_STAGES;
-    if (t_lo >= t_hi) return;       // before anything is allocated, the same for every thread
-
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&s_tmem)), "n"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
@@ -77,6 +76,7 @@ __global__ void __launch_bounds__(192, 1) conv3_wgrad_kernel(const __grid_consta
     const uint32_t tmem = __reduce_max_sync(0xffffffffu, s_tmem);
 
     bool fault = false;
+    chain_wait();
     if (warp == 4) {
         const uint32_t lead = elect_lead();
         RollRing st(stages);

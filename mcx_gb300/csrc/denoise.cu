@@ -437,6 +437,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
+// A kernel launched by launch_chained may start while the one before it on the stream still runs: it touches nothing but its
+// own shared and tensor memory until chain_wait, which returns once that one has finished and its writes are seen.
+// Every thread calls it, so that a kernel's end means the end of all before it.  chain_next lets the next such
+// kernel start as this one's CTAs leave.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
@@ -630,7 +637,9 @@ __device__ __forceinline__ void store8(bf16* p, const float (&f)[8]) {
 // block adds its rows through shared memory, one atomic a channel and block.  Bound by the read of dY: 524288 rows of 16
 // channels (17 MB) took 18.7 us with 2-byte loads, one channel a
 // thread and 128 blocks, and take 6.3.
-__global__ void __launch_bounds__(256) bias_grad8_kernel(const bf16* __restrict__ dy, float* __restrict__ db, long long m, int c) {
+__global__ void __launch_bounds__(256) bias_grad8_kernel(const bf16* dy, float* db, long long m, int c) {
+    chain_next();
+    chain_wait();
     __shared__ float part[256][9];
     const int cc = c / 8, rows = 256 / cc;
     const int ch = threadIdx.x % cc, r0 = threadIdx.x / cc;
@@ -654,7 +663,9 @@ __global__ void __launch_bounds__(256) bias_grad8_kernel(const bf16* __restrict_
 
 // 2x2x2 average pooling; (d, h, w) are the fine grid's sizes.  One thread per coarse voxel and
 // 8-channel chunk.
-__global__ void pool_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, int nvol, int d, int h, int w, int c) {
+__global__ void pool_kernel(const bf16* x, bf16* y, int nvol, int d, int h, int w, int c) {
+    chain_next();
+    chain_wait();
     const int d2 = d / 2, h2 = h / 2, w2 = w / 2, cc = c / 8;
     long long total = (long long)nvol * d2 * h2 * w2 * cc;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total; q += (long long)gridDim.x * blockDim.x) {
@@ -691,10 +702,11 @@ struct FastDiv {
 // block apart, all four read before the first is written, their places found with 32-bit multiplications.  Bound by the
 // write: 128^3 of 32 + 16 channels (84 MB read, 201 MB written) in 43 us, 6.6 TB/s (a chunk
 // at a time, 64-bit divisions: 98).
-__global__ void __launch_bounds__(256) upcat4_kernel(const uint4* __restrict__ low, const uint4* __restrict__ skip,
-                                                     uint4* __restrict__ cat, unsigned total, unsigned k1, FastDiv ct, FastDiv w,
-                                                     FastDiv h, FastDiv d) {
+__global__ void __launch_bounds__(256) upcat4_kernel(const uint4* low, const uint4* skip, uint4* cat, unsigned total,
+                                                     unsigned k1, FastDiv ct, FastDiv w, FastDiv h, FastDiv d) {
     const unsigned q0 = blockIdx.x * 1024u + threadIdx.x, k2 = ct.d - k1;
+    chain_next();
+    chain_wait();
     uint4 u[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -704,9 +716,9 @@ __global__ void __launch_bounds__(256) upcat4_kernel(const uint4* __restrict__ l
         if (ch < k1) {
             const unsigned yz = w.div(v), x = v - yz * w.d, zn = h.div(yz), y = yz - zn * h.d, n = d.div(zn), z = zn - n * d.d;
             const unsigned pv = ((n * (d.d >> 1) + (z >> 1)) * (h.d >> 1) + (y >> 1)) * (w.d >> 1) + (x >> 1);
-            u[i] = __ldg(low + (size_t)pv * k1 + ch);
+            u[i] = low[(size_t)pv * k1 + ch];
         } else {
-            u[i] = __ldcs(skip + (size_t)v * k2 + (ch - k1));
+            u[i] = skip[(size_t)v * k2 + (ch - k1)];
         }
     }
 #pragma unroll
@@ -789,13 +801,12 @@ __global__ void unpool_add_kernel(const bf16* __restrict__ dpool, const bf16* __
 
 // Head: out[v] = xres[v] + b + sum_c w[c] * act[v, c] (16 channels).  With a target, also the
 // masked L1 loss, dact = g * w * (act > 0), dw += g * act, db += g, g = sign(out - t) * valid * inv.
-__global__ void __launch_bounds__(256) head_kernel(const bf16* __restrict__ act, const float* __restrict__ xres,
-                                                   const float* __restrict__ w, const float* __restrict__ b,
-                                                   const float* __restrict__ target, const float* __restrict__ valid,
-                                                   float* __restrict__ out, bf16* __restrict__ dact,
-                                                   float* __restrict__ dw, float* __restrict__ db,
-                                                   float* __restrict__ loss, long long m, float inv) {
+__global__ void __launch_bounds__(256) head_kernel(const bf16* act, const float* xres, const float* w, const float* b,
+                                                   const float* target, const float* valid, float* out, bf16* dact, float* dw,
+                                                   float* db, float* loss, long long m, float inv) {
     __shared__ float red[8][18];
+    chain_next();
+    chain_wait();
     float gw[16], gb = 0.f, ls = 0.f;
 #pragma unroll
     for (int c = 0; c < 16; ++c) gw[c] = 0.f;
@@ -1042,6 +1053,25 @@ int launched() {
     return 0;
 }
 
+// A launch that may overlap the end of the kernel before it on the stream (chain_wait in the kernel holds it back).  The
+// network is two dozen kernels of 5 to 120 us: their launches, barriers and tensor memory set up behind the one before took
+// a 128^3 forward pass from 633 to FORWARD_FIGURE us, a convolution of a row of its kind from 46.3 to 42.9 (16 to 16).
+template <class... P, class... A>
+int launch_chained(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    return launched();
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 int grid_for(long long work, int block) {
@@ -1156,9 +1186,8 @@ int conv3_roll_launch(const bf16* x, const bf16* w, const float* bias, const bf1
     const int grid = (int)(planes < sms ? planes : sms);
     const int chunk = TAPS || slices == 1 ? g.d : S::R;
     const bool wide = ((reinterpret_cast<uintptr_t>(y)) & 31u) == 0;
-    kern<<<grid, 320, smem, st>>>(xmap, wmap, bias, mask, y, g, cin, cout, relu, tx, ty, (int)planes, chunk, stages, wbufs,
-                                  wide ? 1 : 0);
-    return launched();
+    return launch_chained(kern, (unsigned)grid, 320, smem, st, xmap, wmap, bias, mask, y, g, cin, cout, relu, tx, ty, (int)planes,
+                          chunk, stages, wbufs, wide ? 1 : 0);
 }
 
 // Estimated cycles of a CTA's run of conv3_roll_kernel<bn>: its MMAs (the larger of 3027 multiply-adds and 80 operand
@@ -1254,9 +1283,8 @@ int conv3_stream_launch(const bf16* x, const bf16* w, const float* bias, const b
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int smem = wbufs * S::WCHUNK + planes;
     cudaFuncSetAttribute(conv3_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    conv3_stream_kernel<<<(unsigned)(tiles < sms ? tiles : sms), 224, smem, st>>>(
-        xmap, wmap, bias, mask, y, g, cin, cout, relu, tx, ty, (int)tiles, wbufs, (reinterpret_cast<uintptr_t>(y) & 31u) == 0 ? 1 : 0);
-    return launched();
+    return launch_chained(conv3_stream_kernel, (unsigned)(tiles < sms ? tiles : sms), 224, smem, st, xmap, wmap, bias, mask, y, g, cin,
+                          cout, relu, tx, ty, (int)tiles, wbufs, (reinterpret_cast<uintptr_t>(y) & 31u) == 0 ? 1 : 0);
 }
 
 // Narrow 3x3x3 layers run on tcgen05 unless MCXG_DN_MMA_SYNC=1 selects the warp-level mma.sync
@@ -1330,14 +1358,13 @@ int conv3_wgrad_launch(const bf16* dy, const bf16* x, float* dw, Geo g, int cin,
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int parts = sms / groups;
     if (parts < 1) parts = 1;
-    if (parts > tiles) parts = (int)tiles;
+    if (parts > tiles) parts = (int)tiles;          // no run without a tile: the kernel adds what its run left
     int smem = stages * stage;
     if (smem < 120 * 1024) smem = 120 * 1024;       // one CTA an SM: each takes all of its tensor memory
     auto kern = conv3_wgrad_kernel<COUT>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    kern<<<groups * parts, 192, smem, st>>>(maps[0], maps[1], dw, g, cin, tx, ty, tz, (int)tiles, parts, stages,
-                                            (reinterpret_cast<uintptr_t>(dw) & 15u) == 0 ? 1 : 0);
-    return launched();
+    return launch_chained(kern, (unsigned)(groups * parts), 192, smem, st, maps[0], maps[1], dw, g, cin, tx, ty, tz, (int)tiles, parts,
+                          stages, (reinterpret_cast<uintptr_t>(dw) & 15u) == 0 ? 1 : 0);
 }
 
 template <int BM>
@@ -1455,9 +1482,8 @@ int mcxg_dn_bias_grad(const void* dy, float* db, long long m, int c, void* strea
     if (c % 8 == 0 && aligned16(dy)) {
         // about eight rows a thread, at most four blocks an SM
         const long long rows = 256 / (c / 8), want = (m + 8 * rows - 1) / (8 * rows);
-        bias_grad8_kernel<<<(unsigned)(want < 608 ? want : 608), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const bf16*>(dy), db, m, c);
-        return launched();
+        return launch_chained(bias_grad8_kernel, (unsigned)(want < 608 ? want : 608), 256, 0, static_cast<cudaStream_t>(stream),
+                              static_cast<const bf16*>(dy), db, m, c);
     }
     long long rows = 4096;
     unsigned blocks = (unsigned)((m + rows - 1) / rows);
@@ -1468,9 +1494,8 @@ int mcxg_dn_bias_grad(const void* dy, float* db, long long m, int c, void* strea
 int mcxg_dn_pool(const void* x, void* y, int nvol, int d, int h, int w, int c, void* stream) {
     if (!x || !y || !dims_ok(nvol, d, h, w) || (d | h | w) & 1 || c % 8) return fail("pool: bad shape");
     long long work = (long long)nvol * (d / 2) * (h / 2) * (w / 2) * (c / 8);
-    pool_kernel<<<grid_for(work, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const bf16*>(x), static_cast<bf16*>(y), nvol, d, h, w, c);
-    return launched();
+    return launch_chained(pool_kernel, (unsigned)grid_for(work, 256), 256, 0, static_cast<cudaStream_t>(stream),
+                          static_cast<const bf16*>(x), static_cast<bf16*>(y), nvol, d, h, w, c);
 }
 
 int mcxg_dn_upcat(const void* low, const void* skip, void* cat, int nvol, int d, int h, int w, int c1, int c2,
@@ -1479,10 +1504,10 @@ int mcxg_dn_upcat(const void* low, const void* skip, void* cat, int nvol, int d,
         return fail("upcat: bad shape");
     long long work = (long long)nvol * d * h * w * ((c1 + c2) / 8);
     if (work > 0 && work < (1LL << 31) - 1024 && c1 >= 0 && c2 >= 0) {
-        upcat4_kernel<<<(unsigned)((work + 1023) / 1024), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const uint4*>(low), static_cast<const uint4*>(skip), static_cast<uint4*>(cat), (unsigned)work,
-            (unsigned)(c1 / 8), FastDiv((unsigned)((c1 + c2) / 8)), FastDiv((unsigned)w), FastDiv((unsigned)h), FastDiv((unsigned)d));
-        return launched();
+        return launch_chained(upcat4_kernel, (unsigned)((work + 1023) / 1024), 256, 0, static_cast<cudaStream_t>(stream),
+                              static_cast<const uint4*>(low), static_cast<const uint4*>(skip), static_cast<uint4*>(cat), (unsigned)work,
+                              (unsigned)(c1 / 8), FastDiv((unsigned)((c1 + c2) / 8)), FastDiv((unsigned)w), FastDiv((unsigned)h),
+                              FastDiv((unsigned)d));
     }
     upcat_kernel<<<grid_for(work, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const bf16*>(low), static_cast<const bf16*>(skip), static_cast<bf16*>(cat), nvol, d, h, w, c1, c2);
@@ -1516,9 +1541,8 @@ int mcxg_dn_head(const void* act, const float* xres, const float* w, const float
     if (!act || !xres || !w || !b || m <= 0) return fail("head: null tensor or no voxels");
     if (target && (!valid || !dact || !dw || !db || !loss)) return fail("head: training needs valid/dact/dw/db/loss");
     if (!target && !out) return fail("head: nothing to write");
-    head_kernel<<<grid_for(m, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const bf16*>(act), xres, w, b, target, valid, out, static_cast<bf16*>(dact), dw, db, loss, m, inv);
-    return launched();
+    return launch_chained(head_kernel, (unsigned)grid_for(m, 256), 256, 0, static_cast<cudaStream_t>(stream),
+                          static_cast<const bf16*>(act), xres, w, b, target, valid, out, static_cast<bf16*>(dact), dw, db, loss, m, inv);
 }
 
 int mcxg_dn_pack(const float* flux, const uint8_t* label, const float* props, const float* log_photons, void* x0,
