@@ -1782,9 +1782,13 @@ cudaError_t launch_transport(const KParams& in, bool reflect, bool savedet, int 
     // need: whole-chunk reservations would leave some warps with two rounds of photons while
     // others have none, and the launch would end on their tail
     if (p.d_nwork < (unsigned long long)grid * (unsigned long long)block * 16ull) p.chunk = 1;
+    // the same for the photons a warp of the plain path's kernel draws ahead, an eighth of a round; below four photons a thread
+    // it draws none (cube, drawing ahead and not: 1e5 photons 1.69 and 1.67 ms, 3e5 2.16 and 2.17, 1e6 3.60 and 3.66)
+    const bool few = p.d_nwork < (unsigned long long)grid * (unsigned long long)block * 4ull;
+    p.ahead = p.chunk > 1 ? 32u : 4u;
     // the caller sized the shared memory for the variant of its parameters: never launch another's
     if (smem_bytes < transport_smem_bytes(p, block, savedet)) return cudaErrorInvalidValue;
-    const void* k = pick(reflect, savedet, transport_mode(p), p.spare > 0u);
+    const void* k = pick(reflect, savedet, transport_mode(p), few);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
     if (e != cudaSuccess) return e;
     void* args[] = {const_cast<KParams*>(&p)};

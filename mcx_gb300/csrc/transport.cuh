@@ -152,6 +152,7 @@ struct KParams {
     unsigned long long seed;
     unsigned long long* work;       // photon counter the persistent warps draw chunks from
     int chunk;                      // photons per warp refill
+    unsigned ahead;                 // plain path: photons a warp draws at a time
     unsigned spare;                 // plain path: lanes of a warp left without a photon
     unsigned int step_cap;          // safety cap on steps per photon (error flag when hit)
 

@@ -42,6 +42,8 @@ struct LeanSmem {
     float4 prop[kMaxMedia];                     // (mua, mus, g, n)
     float2 inv[kMaxMedia];                      // (1 / mus, deposit per absorbed weight)
     unsigned long long pool[2 * kLeanWarps];    // per warp: next, end of its photon-index pool
+    ulonglong2 queue[kLeanBlock];               // per warp: the random states of photons drawn ahead,
+    float qscat[kLeanBlock];                    // and their first scattering lengths
     unsigned wcount[2 * kLeanWarps];            // per warp: launches tried, photons run
     unsigned steps[kLeanBlock];                 // steps of the photons the lane has finished
     unsigned nscat0[kLeanBlock];                // detector runs: the lane's scatter count at the last change of medium
@@ -83,8 +85,8 @@ __device__ __forceinline__ float ahead(float v) { return v > 0.f ? 1.f : 0.f; }
 template <bool AREA>
 constexpr unsigned kLeanTogether = AREA ? 4u : 1u;
 
-// What a launch of the kernel is for: photons by the thousand a warp; few of them, spread over all warps (in the same kernel
-// the spare lanes' arithmetic cost the long runs 1%); a replay.
+// What a launch of the kernel is for: at least four photons a thread; fewer, spread over all warps where they are fewer than
+// its lanes (in the same kernel the spare lanes' arithmetic cost the long runs 1%); a replay.
 enum LeanKind : int { kLeanMany = 0, kLeanFew, kLeanReplays };
 
 template <bool REFLECT, bool SAVEDET, bool AREA, int KIND, int MINB>
@@ -92,7 +94,7 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
     extern __shared__ __align__(16) unsigned char smem_raw[];
     LeanSmem& S = *reinterpret_cast<LeanSmem*>(smem_raw);
     constexpr unsigned B = kLeanBlock, kTogether = kLeanTogether<AREA>;
-    constexpr bool REPLAY = KIND == kLeanReplays;
+    constexpr bool REPLAY = KIND == kLeanReplays, QUEUE = KIND == kLeanMany && !AREA && !SAVEDET && !REFLECT;
     const unsigned spare = KIND == kLeanMany ? 0u : P.spare;        // lanes left without a photon
     unsigned* const tile = reinterpret_cast<unsigned*>(S.ppath) + (SAVEDET ? P.partialdata * B : 0u);
     const unsigned tid = threadIdx.x;
@@ -141,6 +143,7 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
     int rbin = -1;                      // replay: its field block (gate + detector offset), -1 none
     unsigned c_scat = 0u, c_dep = 0u, c_tile = 0u;
     S.steps[tid] = 0u;
+    unsigned q_next = 0u, q_left = 0u;  // warp-uniform: photons drawn ahead
     // the step cap ends a photon 1023 steps past it, the latest transport_kernel does
     const unsigned limit = P.step_cap < 0xFFFFFC00u ? P.step_cap + 1023u : 0xFFFFFFFFu;
 
@@ -183,47 +186,88 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
                 const unsigned want = ~live;
                 const unsigned cnt = idle - spare;
                 const unsigned rank = __popc(want & ((1u << lane) - 1u));
-                unsigned long long pool_next = S.pool[2 * warp], pool_end = S.pool[2 * warp + 1];
-                const unsigned long long avail = pool_end - pool_next;
-                unsigned long long mine = pool_next + rank;
-                if (avail < cnt) {
-                    // reserve at least what the dead lanes need, normally a whole chunk
-                    const unsigned long long take = max((unsigned long long)P.chunk, (unsigned long long)(cnt - avail));
-                    unsigned long long base = 0ull;
-                    if (lane == 0) base = atomicAdd(P.work, take);
-                    base = __shfl_sync(kFull, base, 0);
-                    if (rank >= avail) mine = base + (rank - avail);
-                    pool_next = base + (cnt - avail);
-                    pool_end = base + take;
-                    if (base >= P.d_nwork) refill_at = kNever;
+                bool start;
+                float first = 0.f;
+                if constexpr (QUEUE) {
+                    // A lane of a pencil's warp dies every six steps or so, and all wait for its relaunch: the seeding and
+                    // the first flight are drawn for up to 32 photons at a time, a lane each (cube, 8e6 photons 16.5 ->
+                    // 15.9 ms, 1e6 3.66 -> 3.60).  Not with an area source, whose kernel spills more with it (26.9 -> 27.2
+                    // on the planar source at 8e6), nor with detector records (two media, 3e5: 4.05 -> 4.14) or reflection
+                    // (layered head, 1e6: 25.0 -> 25.5), where a photon lives longer and the registers are fewer.
+                    if (q_left == 0u) {
+                        const unsigned take = max(cnt, P.ahead);
+                        unsigned long long base = 0ull;
+                        if (lane == 0) base = atomicAdd(P.work, (unsigned long long)take);
+                        base = __shfl_sync(kFull, base, 0);     // and every lane has read the entries before
+                        if (lane < take && base + lane < P.d_nwork) {
+                            ulonglong2 q;
+                            seed_photon(P.seed, P.photon_offset + base + lane, q.x, q.y);
+                            // the launch flight takes the first of its step's three numbers
+                            float u_len, u_phi, u_th;
+                            rng_next3(q.x, q.y, u_len, u_phi, u_th);
+                            S.qscat[tid] = -__logf(u_len + kEPS);
+                            S.queue[tid] = q;
+                        }
+                        q_next = tid - lane;
+                        q_left = base >= P.d_nwork ? 0u : (unsigned)min((unsigned long long)take, P.d_nwork - base);
+                        if (q_left == 0u) refill_at = kNever;
+                        __syncwarp();
+                    }
+                    start = !alive && rank < q_left;
+                    if (start) {
+                        const ulonglong2 q = S.queue[q_next + rank];
+                        r0 = q.x;
+                        r1 = q.y;
+                        first = S.qscat[q_next + rank];
+                    }
+                    const unsigned taken = min(cnt, q_left);
+                    q_next += taken;
+                    q_left -= taken;
                 } else {
-                    pool_next += cnt;
+                    unsigned long long pool_next = S.pool[2 * warp], pool_end = S.pool[2 * warp + 1];
+                    const unsigned long long avail = pool_end - pool_next;
+                    unsigned long long mine = pool_next + rank;
+                    if (avail < cnt) {
+                        // reserve at least what the dead lanes need, normally a whole chunk
+                        const unsigned long long take = max((unsigned long long)P.chunk, (unsigned long long)(cnt - avail));
+                        unsigned long long base = 0ull;
+                        if (lane == 0) base = atomicAdd(P.work, take);
+                        base = __shfl_sync(kFull, base, 0);
+                        if (rank >= avail) mine = base + (rank - avail);
+                        pool_next = base + (cnt - avail);
+                        pool_end = base + take;
+                        if (base >= P.d_nwork) refill_at = kNever;
+                    } else {
+                        pool_next += cnt;
+                    }
+                    __syncwarp();               // every lane has read the pool before lane 0 rewrites it
+                    if (lane == 0) {
+                        S.pool[2 * warp] = pool_next;
+                        S.pool[2 * warp + 1] = pool_end;
+                    }
+                    __syncwarp();               // and reads the new one at the next refill
+                    start = !alive && mine < P.d_nwork && (KIND == kLeanMany || rank < cnt);
+                    if (start) {
+                        if constexpr (REPLAY) {
+                            // a detected photon again: its saved launch state and detection record
+                            // (src/mcx_core.cu:1203-1211)
+                            r0 = __ldg(P.replay_seed + 2 * mine);
+                            r1 = __ldg(P.replay_seed + 2 * mine + 1);
+                            const float tof = __ldg(P.replay_tof + mine);
+                            rbin = (int)floorf((tof - P.twin0) * P.Rtstep);
+                            if (rbin < 0 || rbin >= P.maxgate) rbin = -1;      // detected outside this gate group
+                            else if (P.replaydet == -1) rbin += ((__ldg(P.replay_detid + mine) & 0xFFFF) - 1) * P.maxgate;
+                            rw = __ldg(P.replay_w + mine);
+                            if (P.outputtype == kOutWLTOF) rtof = tof;
+                            // the draw by which the recorded run picked its source (src/mcx_core.cu:1229-1231)
+                            if (P.srcid >= 1) (void)rng_next(r0, r1);
+                        } else {
+                            seed_photon(P.seed, P.photon_offset + mine, r0, r1);
+                        }
+                    }
                 }
-                __syncwarp();               // every lane has read the pool before lane 0 rewrites it
-                if (lane == 0) {
-                    S.pool[2 * warp] = pool_next;
-                    S.pool[2 * warp + 1] = pool_end;
-                }
-                __syncwarp();               // and reads the new one at the next refill
-                const bool start = !alive && mine < P.d_nwork && (KIND == kLeanMany || rank < cnt);
                 bool entered = false;
                 if (start) {
-                    if constexpr (REPLAY) {
-                        // a detected photon again: its saved launch state and detection record
-                        // (src/mcx_core.cu:1203-1211)
-                        r0 = __ldg(P.replay_seed + 2 * mine);
-                        r1 = __ldg(P.replay_seed + 2 * mine + 1);
-                        const float tof = __ldg(P.replay_tof + mine);
-                        rbin = (int)floorf((tof - P.twin0) * P.Rtstep);
-                        if (rbin < 0 || rbin >= P.maxgate) rbin = -1;      // detected outside this gate group
-                        else if (P.replaydet == -1) rbin += ((__ldg(P.replay_detid + mine) & 0xFFFF) - 1) * P.maxgate;
-                        rw = __ldg(P.replay_w + mine);
-                        if (P.outputtype == kOutWLTOF) rtof = tof;
-                        // the draw by which the recorded run picked its source (src/mcx_core.cu:1229-1231)
-                        if (P.srcid >= 1) (void)rng_next(r0, r1);
-                    } else {
-                        seed_photon(P.seed, P.photon_offset + mine, r0, r1);
-                    }
                     if (!AREA || P.srctype == kSrcPencil) {
                         // the pencil's launch state, traced through the void by the host
                         px = P.src_p.x; py = P.src_p.y; pz = P.src_p.z; w = P.src_p.w;
@@ -252,10 +296,14 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
                         const float2 iv = S.inv[lab & kLabelMask];
                         mua = pr.x; mus = pr.y; n = pr.w; n1 = pr.w;
                         rmus = iv.x; rmua = iv.y;
-                        // the launch flight takes the first of its step's three numbers
-                        float u_len, u_phi, u_th;
-                        rng_next3(r0, r1, u_len, u_phi, u_th);
-                        pscat = -__logf(u_len + kEPS);
+                        if (QUEUE) {
+                            pscat = first;
+                        } else {
+                            // the launch flight takes the first of its step's three numbers
+                            float u_len, u_phi, u_th;
+                            rng_next3(r0, r1, u_len, u_phi, u_th);
+                            pscat = -__logf(u_len + kEPS);
+                        }
                         S.wlaunch[tid] = w;
                         w0 = w;
                         eabs = 0.f;

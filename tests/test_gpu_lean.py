@@ -38,6 +38,9 @@ DECKS = {
     "one photon": lambda: problems.workload0(1),
     "a warp and one": lambda: problems.workload0(33),
     "cube": lambda: problems.workload0(300_000),
+    "photons drawn ahead": lambda: problems.workload0(700_001),
+    "photons drawn a warp ahead": lambda: problems.workload0(2_000_033),
+    "drawn ahead among indices and a void": lambda: _mixed(700_001, isreflect=0, issavedet=0),
     "sphere, gates, detectors": lambda: problems.workload1(200_000),
     "void to skip": lambda: problems.workload2(50_000, n=64),
     "indices and a void": lambda: _mixed(200_000),
