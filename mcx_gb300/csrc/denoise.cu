@@ -79,15 +79,6 @@ struct Geo {
     long long m;  // voxels over all volumes
 };
 
-// Neighbour of voxel (z, y, x) at tap t of a 3x3x3 stencil (t = dz*9 + dy*3 + dx), or -1 outside.
-__device__ __forceinline__ long long tap_voxel(const Geo& g, long long v, int z, int y, int x, int t, int taps) {
-    if (taps == 1) return v;
-    int dz = t / 9 - 1, dy = (t / 3) % 3 - 1, dx = t % 3 - 1;
-    int zz = z + dz, yy = y + dy, xx = x + dx;
-    if (zz < 0 || zz >= g.d || yy < 0 || yy >= g.h || xx < 0 || xx >= g.w) return -1;
-    return v + (long long)dz * g.h * g.w + dy * g.w + dx;
-}
-
 // ---------------------------------------------------------------------------------------------
 // Forward convolution (and data gradient): Y[v, n0:n0+BN] over a tile of BM voxels.  K runs over
 // (tap, input channel) flattened, k = tap*cin + ci, in stages of BK: with few input channels one
@@ -633,30 +624,47 @@ __device__ __forceinline__ void store8(bf16* p, const float (&f)[8]) {
     *reinterpret_cast<uint4*>(p) = u;
 }
 
-// The same for channels in whole 16-byte chunks: a thread keeps one chunk of 8 channels and walks rows a grid apart, the
-// block adds its rows through shared memory, one atomic a channel and block.  Bound by the read of dY: 524288 rows of 16
-// channels (17 MB) took 18.7 us with 2-byte loads, one channel a
-// thread and 128 blocks, and take 6.3.
+// The same for channels in whole 16-byte chunks: a thread keeps one chunk of 8 channels and walks rows a grid apart, four in
+// flight, the block adds its rows by shuffles and through shared memory, one atomic a channel and block.  Bound by the read of
+// dY and a launch: 524288 rows of 16 channels (17 MB) took 18.7 us with 2-byte loads, one channel a thread and 128 blocks,
+// 6.3 with a row in flight and a thread adding a channel's 128 partial sums, and take 4.3.
 __global__ void __launch_bounds__(256) bias_grad8_kernel(const bf16* dy, float* db, long long m, int c) {
     chain_next();
     chain_wait();
-    __shared__ float part[256][9];
+    __shared__ float part[8][256];
     const int cc = c / 8, rows = 256 / cc;
     const int ch = threadIdx.x % cc, r0 = threadIdx.x / cc;
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (long long v = (long long)blockIdx.x * rows + r0; v < m; v += (long long)gridDim.x * rows) {
-        float f[8];
-        load8(dy + v * c + ch * 8, f);
+    const long long step = (long long)gridDim.x * rows;
+    for (long long v = (long long)blockIdx.x * rows + r0; v < m; v += 4 * step) {
+        float f[4][8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) s[e] += f[e];
+        for (int i = 0; i < 4; ++i) {           // four rows in flight
+            if (v + i * step < m) {
+                load8(dy + (v + i * step) * c + ch * 8, f[i]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[i][e] = 0.f;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) s[e] += f[i][e];
     }
+    // over the warp's lanes of one chunk (cc is a power of two of at most 32), then over the warps
+    for (int o = cc; o < 32; o *= 2)
 #pragma unroll
-    for (int e = 0; e < 8; ++e) part[threadIdx.x][e] = s[e];
+        for (int e = 0; e < 8; ++e) s[e] += __shfl_xor_sync(0xffffffffu, s[e], o);
+    if ((int)(threadIdx.x & 31) < cc) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) part[threadIdx.x / 32][ch * 8 + e] = s[e];
+    }
     __syncthreads();
     if ((int)threadIdx.x < c) {
-        const int k = threadIdx.x / 8, e = threadIdx.x % 8;
         float t = 0.f;
-        for (int r = 0; r < rows; ++r) t += part[r * cc + k][e];
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += part[w][threadIdx.x];
         atomicAdd(db + threadIdx.x, t);
     }
 }
