@@ -51,14 +51,13 @@ CPU_SAMPLE = {"workload0": 8_000_000, "workload1": 4_000_000, "workload2": 1_000
 CONTEST_DECKS = ("cube60", "cube60b", "cube60planar")
 
 # Thread-level instructions per transport step (ncu smsp__inst_executed.sum x
-# smsp__thread_inst_executed_per_inst_executed.ratio over the kernel's own step counter) and
-# DRAM bytes of one launch (dram__bytes_read.sum + dram__bytes_write.sum), from one ncu capture
-# of `bench.py --workload W --photons 20000000 --steps 1 --warmup 1`.  The DRAM bytes are the
-# field's first read and its write-back: the field and labels stay in L2, so they do not grow
-# with the photon count.
-# workload2: `bench.py --workload workload2 --photons 2000000 --steps 1 --warmup 1 --no-cpu-baseline`,
-# the timed launch (-s 7 -c 1): 5.382e10 warp instructions x 15.63 lanes over 2e6 x 1606.5 steps.
-NCU_PER_STEP = {"workload0": 222.8, "workload1": 272.0, "workload2": 261.8}
+# smsp__thread_inst_executed_per_inst_executed.ratio over the kernel's own step counter), one ncu
+# capture of lean_kernel per deck (8e6, 8e6 and 1e6 photons), and DRAM bytes of one launch
+# (dram__bytes_read.sum + dram__bytes_write.sum), from one ncu capture
+# of `bench.py --workload W --photons 20000000 --steps 1 --warmup 1` (workload2: 2000000).  The DRAM
+# bytes are the field's first read and its write-back: the field and labels stay in L2, so they do
+# not grow with the photon count.
+NCU_PER_STEP = {"workload0": 166.6, "workload1": 177.8, "workload2": 174.1}
 NCU_DRAM_PER_LAUNCH = {"workload0": 1.63e6, "workload1": 41.59e6, "workload2": 25.97e6}
 
 

@@ -29,9 +29,9 @@
 // tap), else they cycle through a ring of slice buffers.  Every wait is bounded: one that gives up sets g_dn_fault, and
 // the CTA still releases its tensor memory and returns.
 //
-// Measured (GB300, us, the kernel before -> this one): 16 -> 16 at 128^3 77 -> 46; 48 -> 16 206 -> 120; 16 -> 48 206 -> 62
-// (1390 TFLOP/s, 73% of the measured peak); 32 -> 32 at 64^3 33 -> 19; 96 -> 32 82 -> 43; 64 -> 64 at 4 x 32^3 134 -> 36;
-// 64 -> 192 at 32^3 115 -> 28; 128 -> 128 at 16^3 72 -> 19.  What bounds it: operand reads, about 80 bytes a cycle
+// Measured (GB300, us, the kernel before -> this one): 16 -> 16 at 128^3 77 -> 42; 48 -> 16 206 -> 117; 16 -> 48 206 -> 60
+// (1460 TFLOP/s, 77% of the measured peak); 32 -> 32 at 64^3 33 -> 17; 96 -> 32 82 -> 40; 64 -> 64 at 4 x 32^3 134 -> 34;
+// 64 -> 192 at 32^3 115 -> 25; 128 -> 128 at 16^3 72 -> 15 (back to back, launches overlapping).  What bounds it: operand reads, about 80 bytes a cycle
 // (70 cycles per MMA of N = 48), up to N = 144; the math at N = 192; beyond that a fixed 5 us (launch, tensor
 // memory, first weights and halo).
 

@@ -1063,7 +1063,7 @@ int launched() {
 
 // A launch that may overlap the end of the kernel before it on the stream (chain_wait in the kernel holds it back).  The
 // network is two dozen kernels of 5 to 120 us: their launches, barriers and tensor memory set up behind the one before took
-// a 128^3 forward pass from 633 to 585 us, a convolution of a row of its kind from 46.3 to 42.9 (16 to 16).
+// a 128^3 forward pass from 633 to 585 us, a convolution in a row of its kind from 46.3 to 42.5 (16 to 16 at 128^3).
 template <class... P, class... A>
 int launch_chained(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchAttribute attr{};

@@ -24,8 +24,8 @@
 //     them cost 12 of 179 thread instructions a step (17.1 -> 16.5 ms on the cube at 8e6 photons).
 // Measured, kernel time in transport_kernel and here (GB300, 2070 MHz): sphere with 50 gates and four
 // detectors, 2e6 photons, 18.4 -> 11.8 ms; layered 128^3 head, 3e5, 43.3 -> 18.7; planar source, 1e6, 9.24 ->
-// 5.20; homogeneous cube, 2e6, 7.99 -> 5.65 and 1e4 photons, 2.86 -> 1.45.  On the cube 167 thread instructions
-// a step instead of 223, 15.6 lanes an instruction, 82% of the issue slots: what binds it is issue still, the
+// 5.20; homogeneous cube, 2e6, 7.96 -> 5.42 and 1e4 photons, 2.84 -> 1.23.  On the cube 167 thread instructions
+// a step instead of 223, 16 lanes an instruction, 83% of the issue slots: what binds it is issue still, the
 // scattering and the crossing block each run by the half of the lanes that need it.
 //
 // REPLAY runs detected photons again from their saved states into the Jacobian of absorption (or its time-of-flight
