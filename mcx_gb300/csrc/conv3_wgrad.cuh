@@ -42,9 +42,43 @@ __device__ __forceinline__ uint64_t umma_desc_mn32(uint32_t saddr, uint32_t lbo,
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (6ull << 61);
 }
 
+// The sums of a CTA's group over its run, voxel by voxel: for a run that holds an infinity or a NaN (below).
+template <int COUT>
+__device__ __noinline__ void wgrad_by_voxel(const bf16* dy, const bf16* x, float* dw, const Geo& g, int cin, int tiles_x, int tiles_y,
+                                            int tiles_z, int t_lo, int t_hi, int pair0, int pairs) {
+    constexpr int PZ = WgradShape<COUT>::PZ;
+    for (int o = threadIdx.x; o < pairs * 3 * COUT * 16; o += blockDim.x) {
+        const int ci = o % 16, co = o / 16 % COUT, dz = o / (16 * COUT) % 3, pair = pair0 + o / (48 * COUT);
+        const int tap = pair % 9, cx = pair / 9 * 16 + ci;
+        float sum = 0.f;
+        for (int t = t_lo; t < t_hi; ++t) {
+            int r = t;
+            const int x0 = (r % tiles_x) * 8;
+            r /= tiles_x;
+            const int y0 = (r % tiles_y) * 16;
+            r /= tiles_y;
+            const int z0 = (r % tiles_z) * PZ, n = r / tiles_z;
+            float s = 0.f;
+            for (int z = z0; z < min(z0 + PZ, g.d); ++z)
+                for (int y = y0; y < min(y0 + 16, g.h); ++y)
+                    for (int xx = x0; xx < min(x0 + 8, g.w); ++xx) {
+                        const int uz = z + dz - 1, uy = y + tap / 3 - 1, ux = xx + tap % 3 - 1;
+                        const bool in = (unsigned)uz < (unsigned)g.d && (unsigned)uy < (unsigned)g.h && (unsigned)ux < (unsigned)g.w;
+                        const float a = __bfloat162float(dy[(((long long)n * g.d + z) * g.h + y) * g.w * COUT + (long long)xx * COUT + co]);
+                        const float b =
+                            in ? __bfloat162float(x[((((long long)n * g.d + uz) * g.h + uy) * g.w + ux) * cin + cx]) : 0.f;
+                        s = fmaf(a, b, s);
+                    }
+            sum += s;
+        }
+        atomicAdd(dw + ((long long)co * 27 + dz * 9 + tap) * cin + cx, sum);
+    }
+}
+
 template <int COUT>
 __global__ void __launch_bounds__(192, 1) conv3_wgrad_kernel(const __grid_constant__ CUtensorMap ymap,
-                                                             const __grid_constant__ CUtensorMap xmap, float* __restrict__ dw, Geo g,
+                                                             const __grid_constant__ CUtensorMap xmap, const bf16* dy,
+                                                             const bf16* x, float* dw, Geo g,
                                                              int cin, int tiles_x, int tiles_y, int tiles_z, int tiles, int parts,
                                                              int stages, int vec4) {
     using S = WgradShape<COUT>;
@@ -145,16 +179,38 @@ __global__ void __launch_bounds__(192, 1) conv3_wgrad_kernel(const __grid_consta
     // the stages are free for the sums once every MMA has read them
     const bool reached = warp_wait(done, 0u), ok = __syncthreads_and(reached) != 0;
     fault |= !reached;
-    if (warp < 4 && ok) {
+    constexpr int CB = PZ > 1 ? 4 : 3;                      // blocks of 16 columns a warp reads of an accumulator
+    const int p_low = PZ > 1 ? (2 * warp) % PZ : 0;
+    bool plain = true;
+    if (ok && (g.w % 8 | g.h % 16 | g.d % PZ) != 0) {
+        // A tile that ends outside the volume pairs zeros of dY there with voxels of X inside it, which adds nothing
+        // but where X holds an infinity or a NaN.  A run with such a sum is added up over the volume's own pairs (the look
+        // at the sums costs no time that shows).
+        bool odd = false;
+        if (warp < 4) {
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            for (int p = 0; p < pairs; ++p) {
+#pragma unroll
+                for (int c = 0; c < CB; ++c) {
+                    uint32_t v[16];
+                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(p * N + (p_low + c) * 16), v);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) odd |= (v[i] & 0x7F800000u) == 0x7F800000u;
+                }
+            }
+        }
+        plain = __syncthreads_or(odd) == 0;
+        if (!plain) wgrad_by_voxel<COUT>(dy, x, dw, g, cin, tiles_x, tiles_y, tiles_z, t_lo, t_hi, pair0, pairs);
+    }
+    if (warp < 4 && ok && plain) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         // lane r holds row r: channel co of plane p, which pairs with the X planes p .. p + 2 (columns 16 p ..)
-        const int r = warp * 32 + lane, p_low = PZ > 1 ? (2 * warp) % PZ : 0;
+        const int r = warp * 32 + lane;
         const bool high = PZ > 1 && lane >= 16;             // the warp's upper half holds the next plane
         const int co = (r >> 4) / PZ * 16 + (r & 15);
         float* const sums = reinterpret_cast<float*>(dyn_smem);         // [4 warps][16][48] where warps share channels
         constexpr int SHARE = PZ >= 8 ? 4 : PZ >= 4 ? 2 : 1;            // warps that hold the same channels
         for (int p = 0; p < pairs; ++p) {
-            constexpr int CB = PZ > 1 ? 4 : 3;              // column blocks to read
             uint32_t v[CB * 16];
 #pragma unroll
             for (int c = 0; c < CB; ++c)

@@ -1371,7 +1371,7 @@ int conv3_wgrad_launch(const bf16* dy, const bf16* x, float* dw, Geo g, int cin,
     if (smem < 120 * 1024) smem = 120 * 1024;       // one CTA an SM: each takes all of its tensor memory
     auto kern = conv3_wgrad_kernel<COUT>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return launch_chained(kern, (unsigned)(groups * parts), 192, smem, st, maps[0], maps[1], dw, g, cin, tx, ty, tz, (int)tiles, parts,
+    return launch_chained(kern, (unsigned)(groups * parts), 192, smem, st, maps[0], maps[1], dy, x, dw, g, cin, tx, ty, tz, (int)tiles, parts,
                           stages, (reinterpret_cast<uintptr_t>(dw) & 15u) == 0 ? 1 : 0);
 }
 

@@ -63,3 +63,35 @@ def test_weight_and_bias_gradient(engine, case):
     assert b[0] == b[-1] == 0.25
     rb = dyT.sum(1) + 0.25
     assert np.abs(b[1:-1] - rb).max() <= 1e-4 * max(1.0, np.abs(rb).max())
+
+
+@pytest.mark.parametrize("case", [(1, 33, 33, 31, 16, 16), (1, 35, 33, 30, 16, 32), (1, 9, 31, 31, 64, 64), (1, 17, 17, 15, 128, 128)],
+                         ids=lambda c: "x".join(map(str, c[:4])) + " %d-%d" % c[4:])
+def test_infinities_stay_with_their_voxels(engine, case):
+    """A tile's padding outside the volume meets voxels inside it: an infinity or a NaN at the volume's faces reaches the taps
+    that pair it with a voxel of the volume, as in the sum over the volume, and no other."""
+    from mcx_gb300._lib import lib
+
+    n, d, h, w, cin, cout = case
+    vox = n * d * h * w
+    rng = np.random.default_rng(sum(case))
+    x = R.bf16(rng.standard_normal((vox, cin)))
+    dy = R.bf16(np.abs(rng.standard_normal((vox, cout))) + 0.1)
+    x5 = x.reshape(n, d, h, w, cin)
+    x5[0, -1, 3, 4, 1], x5[0, 2, -1, 5, 2], x5[0, 4, 5, -1, cin - 1] = np.inf, np.nan, -np.inf
+    X, DY = (torch.from_numpy(a).cuda().to(BF).contiguous() for a in (x, dy))
+    dw = torch.zeros(cout * 27 * cin, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    assert lib.mcxg_dn_conv_wgrad(DY.data_ptr(), X.data_ptr(), dw.data_ptr(), n, d, h, w, cin, cout, 27, st) == 0
+    assert lib.mcxg_dn_check(st) == 0, lib.mcxg_dn_last_error()
+    xp = np.pad(x.astype(np.float64).reshape(n, d, h, w, cin), ((0, 0), (1, 1), (1, 1), (1, 1), (0, 0)))
+    dyT = dy.astype(np.float64).T
+    with np.errstate(invalid="ignore"):
+        ref = np.stack([dyT @ xp[:, t // 9:t // 9 + d, t // 3 % 3:t // 3 % 3 + h, t % 3:t % 3 + w].reshape(vox, cin)
+                        for t in range(27)], 1).reshape(-1)
+    got = dw.cpu().numpy()
+    assert (np.isnan(got) == np.isnan(ref)).all()
+    assert (got[np.isinf(ref)] == ref[np.isinf(ref)]).all()
+    ok = np.isfinite(ref)
+    assert ok.any() and not ok.all()
+    assert np.abs(got[ok] - ref[ok]).max() <= 1e-4 * np.abs(ref[ok]).max()
