@@ -25,6 +25,7 @@
 #include <cudaTypedefs.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -1145,10 +1146,20 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 // Shared memory of conv3_roll_kernel beside its barriers.
 constexpr int kRollSmem = 225 * 1024;
 
+// Lets a kernel have all of kRollSmem, once per device (`done`: a bit each, the kernel's own); asking at every launch cost
+// the small layers, which take 8 us of host time a call, half a microsecond.
+template <class K>
+void allow_smem(K kern, int dev, std::atomic<unsigned long long>& done) {
+    const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
+    if (bit && (done.load(std::memory_order_relaxed) & bit)) return;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRollSmem) == cudaSuccess)
+        done.fetch_or(bit, std::memory_order_relaxed);
+}
+
 // Launch of conv3_roll_kernel for BN output channels a block (BN divides cout).
 template <int BN, bool TAPS>
 int conv3_roll_launch(const bf16* x, const bf16* w, const float* bias, const bf16* mask, bf16* y, Geo g, int cin,
-                      int cout, int relu, int sms, cudaStream_t st) {
+                      int cout, int relu, int dev, int sms, cudaStream_t st) {
     using S = RollShape<BN>;
     auto encode = tensor_map_encoder();
     if (!encode) return fail("conv: cuTensorMapEncodeTiled is not available");
@@ -1190,7 +1201,8 @@ int conv3_roll_launch(const bf16* x, const bf16* w, const float* bias, const bf1
     int smem = wbufs * S::WSLICE + stages * stage;
     if (smem < 120 * 1024) smem = 120 * 1024;
     auto kern = conv3_roll_kernel<BN, TAPS>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static std::atomic<unsigned long long> done{0};
+    allow_smem(kern, dev, done);
     const int grid = (int)(planes < sms ? planes : sms);
     const int chunk = TAPS || slices == 1 ? g.d : S::R;
     const bool wide = ((reinterpret_cast<uintptr_t>(y)) & 31u) == 0;
@@ -1238,8 +1250,8 @@ int conv3_roll_dispatch(const bf16* x, const bf16* w, const float* bias, const b
     }
 #define ROLL(BN)                                                                                            \
     case BN:                                                                                                \
-        return taps ? conv3_roll_launch<BN, true>(x, w, bias, mask, y, g, cin, cout, relu, sms, st)         \
-                    : conv3_roll_launch<BN, false>(x, w, bias, mask, y, g, cin, cout, relu, sms, st)
+        return taps ? conv3_roll_launch<BN, true>(x, w, bias, mask, y, g, cin, cout, relu, dev, sms, st)    \
+                    : conv3_roll_launch<BN, false>(x, w, bias, mask, y, g, cin, cout, relu, dev, sms, st)
     switch (best) {
         ROLL(64);
         ROLL(48);
@@ -1290,7 +1302,8 @@ int conv3_stream_launch(const bf16* x, const bf16* w, const float* bias, const b
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int smem = wbufs * S::WCHUNK + planes;
-    cudaFuncSetAttribute(conv3_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static std::atomic<unsigned long long> done{0};
+    allow_smem(conv3_stream_kernel, dev, done);
     return launch_chained(conv3_stream_kernel, (unsigned)(tiles < sms ? tiles : sms), 224, smem, st, xmap, wmap, bias, mask, y, g, cin,
                           cout, relu, tx, ty, (int)tiles, wbufs, (reinterpret_cast<uintptr_t>(y) & 31u) == 0 ? 1 : 0);
 }
@@ -1370,7 +1383,8 @@ int conv3_wgrad_launch(const bf16* dy, const bf16* x, float* dw, Geo g, int cin,
     int smem = stages * stage;
     if (smem < 120 * 1024) smem = 120 * 1024;       // one CTA an SM: each takes all of its tensor memory
     auto kern = conv3_wgrad_kernel<COUT>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static std::atomic<unsigned long long> done{0};
+    allow_smem(kern, dev, done);
     return launch_chained(kern, (unsigned)(groups * parts), 192, smem, st, maps[0], maps[1], dy, x, dw, g, cin, tx, ty, tz, (int)tiles, parts,
                           stages, (reinterpret_cast<uintptr_t>(dw) & 15u) == 0 ? 1 : 0);
 }

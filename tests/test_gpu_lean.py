@@ -55,6 +55,9 @@ DECKS = {
     "isotropic scattering": lambda: _medium(100_000, [0.005, 1, 0, 1.37]),
     "planar": lambda: problems.cube60planar(200_000),
     "disk": lambda: _mixed(100_000, srctype="disk", srcparam1=[9, 0, 0, 0]),
+    "few photons of a planar source": lambda: problems.cube60planar(5_000),
+    "half a warp's photons of a disk": lambda: _mixed(20_000, srctype="disk", srcparam1=[9, 0, 0, 0]),
+    "few photons, detectors": lambda: _mixed(9_001),
     "isotropic source": lambda: _mixed(100_000, srctype="isotropic", srcpos=[12.3, 14.2, 20.6]),
 }
 
