@@ -736,11 +736,11 @@ struct Session {
         set_transport_variant((o.blocks_per_sm > 0 && o.blocks_per_sm <= 3) ? 3 : 4);
         choose_tile(cfg, o.tile);
         smem = transport_smem_bytes(kp, block, savedet);
-        int bps = transport_blocks_per_sm(reflect, savedet, transport_mode(kp), block, smem);
+        int bps = transport_blocks_per_sm(reflect, savedet, transport_mode(kp, savedet), block, smem);
         if (bps <= 0) {
             kp.tile_on = 0;
             smem = transport_smem_bytes(kp, block, savedet);
-            bps = transport_blocks_per_sm(reflect, savedet, transport_mode(kp), block, smem);
+            bps = transport_blocks_per_sm(reflect, savedet, transport_mode(kp, savedet), block, smem);
         }
         if (bps <= 0) MCXG_RAISE(-6, "the transport kernel does not fit on this device");
         if (o.blocks_per_sm > 0) bps = std::min(bps, o.blocks_per_sm);
@@ -796,11 +796,11 @@ struct Session {
     void apply_tile(int kb) {
         choose_tile(nullptr, kb);
         smem = transport_smem_bytes(kp, block, savedet);
-        int bps = transport_blocks_per_sm(reflect, savedet, transport_mode(kp), block, smem);
+        int bps = transport_blocks_per_sm(reflect, savedet, transport_mode(kp, savedet), block, smem);
         if (bps <= 0) {
             kp.tile_on = 0;
             smem = transport_smem_bytes(kp, block, savedet);
-            bps = transport_blocks_per_sm(reflect, savedet, transport_mode(kp), block, smem);
+            bps = transport_blocks_per_sm(reflect, savedet, transport_mode(kp, savedet), block, smem);
         }
         grid = std::max(1, bps) * sms;
     }
@@ -837,7 +837,7 @@ struct Session {
             kp.mcx_odd = (unsigned)(n - (uint64_t)kp.mcx_per * mcx_streams);
         }
         CK(cudaMemsetAsync(work.p, 0, sizeof(unsigned long long), stream));
-        run_grid = (kp.seed_mode == 1 || fixed_grid) ? grid : transport_grid(kp, grid, block, sms, n);
+        run_grid = (kp.seed_mode == 1 || fixed_grid) ? grid : transport_grid(kp, savedet, grid, block, sms, n);
         kp.spare = transport_spare(run_grid, block, n);
         CK(cudaEventRecord(ev0, stream));
         CK(launch_transport(kp, reflect, savedet, run_grid, block, smem, stream));

@@ -193,11 +193,11 @@ void run_noalloc(const Config* cfg, const uint8_t* d_labels, float* d_field, flo
     // launch shape as the session picks it: without room for the deposit tile, run without it
     const int block = 256;
     size_t smem = transport_smem_bytes(k, block, savedet);
-    int bps = transport_blocks_per_sm(reflect, savedet, transport_mode(k), block, smem);
+    int bps = transport_blocks_per_sm(reflect, savedet, transport_mode(k, savedet), block, smem);
     if (bps <= 0 && k.tile_on) {
         k.tile_on = 0;
         smem = transport_smem_bytes(k, block, savedet);
-        bps = transport_blocks_per_sm(reflect, savedet, transport_mode(k), block, smem);
+        bps = transport_blocks_per_sm(reflect, savedet, transport_mode(k, savedet), block, smem);
     }
     if (bps <= 0) MCXG_RAISE(-6, "the transport kernel does not fit on this device");
     NCK(launch_transport(k, reflect, savedet, bps * sms, block, smem, stream));

@@ -1619,19 +1619,23 @@ __global__ void merge_add_kernel(float* __restrict__ host, const float* __restri
 }  // namespace
 
 // The plain path (transport_lean.cuh): what its kernel leaves out must be off.  No photon reaches
-// gscatter scattering events when that is past the step cap (checked every 1024 steps).
-static bool lean_path(const KParams& p) {
-    return p.seed_mode == 0 && !p.field64 && p.save2pt && !(p.minenergy > 0.f) && p.gscatter > (float)p.step_cap + 2048.f;
+// gscatter scattering events when that is past the step cap (checked every 1024 steps).  Its shared memory
+// beside the tile, which a launch can do without, must fit: its fixed arrays are 7 KB more than the general
+// kernel's at 256 threads and do not shrink with the block, so detector runs of very many media stay there.
+static bool lean_path(const KParams& p, bool savedet) {
+    return p.seed_mode == 0 && !p.field64 && p.save2pt && !(p.minenergy > 0.f) && p.gscatter > (float)p.step_cap + 2048.f &&
+           lean_smem_bytes(p, savedet, false) <= kSmemPerCta;
 }
 
 size_t transport_smem_bytes(const KParams& p, int block, bool savedet) {
-    if (transport_mode(p) >= kLeanPencil) return lean_smem_bytes(p, savedet);
+    const int mode = transport_mode(p, savedet);
+    if (mode >= kLeanPencil) return lean_smem_bytes(p, savedet, p.tile_on);
     size_t b = sizeof(float4) * (size_t)p.medianum;
     b += (2 * sizeof(unsigned long long) + sizeof(int) + 3 * sizeof(unsigned)) * (size_t)(block / 32);
     b += 4 * sizeof(unsigned) * (size_t)block;
     b += sizeof(float) * kNumEnergy * (size_t)block;
     if (savedet) b += sizeof(float) * (size_t)p.partialdata * block;
-    if (transport_mode(p) >= 2) b += 8 + (2 * sizeof(unsigned long long) + 12 * sizeof(float)) * (size_t)block;
+    if (mode >= 2) b += 8 + (2 * sizeof(unsigned long long) + 12 * sizeof(float)) * (size_t)block;
     if (p.tile_on) b += sizeof(unsigned) * (size_t)p.tnx * p.tny * p.tnz * p.tng;
     return b;
 }
@@ -1644,19 +1648,17 @@ static int g_minb = 4;   // register budget of the pencil variants (set by the l
 void set_transport_variant(int minb) { g_minb = (minb == 3) ? 3 : 4; }
 int transport_variant() { return g_minb; }
 
-bool transport_general(const KParams& p) { return transport_mode(p) != 0; }
-
-int transport_mode(const KParams& p) {
+int transport_mode(const KParams& p, bool savedet) {
     if (p.mediaformat == kMedia2LabelSplit) return 4;
     if (media_words(p.mediaformat)) return 3;
     if (p.saveseed || p.traj || p.polarized || p.saveref || p.srcnum > 1 || p.nphase > 2 || p.nangle > 0 || p.nextra > 0) return 2;
     // (the replay outputs at scattering events, and the complex one, need the general kernel's state; sampled sources
     // and a replay into flux run there too)
-    if (p.replay && (p.outputtype == kOutJacobian || p.outputtype == kOutWLTOF) && p.srctype == kSrcPencil && lean_path(p))
+    if (p.replay && (p.outputtype == kOutJacobian || p.outputtype == kOutWLTOF) && p.srctype == kSrcPencil && lean_path(p, savedet))
         return kLeanReplay;
     if (p.replay || p.outputtype > kOutEnergy) return 2;
     const int area = (p.srctype != kSrcPencil) ? 1 : 0;
-    return lean_path(p) ? kLeanPencil + area : area;
+    return lean_path(p, savedet) ? kLeanPencil + area : area;
 }
 
 template <int M, int K>
@@ -1704,10 +1706,10 @@ int transport_blocks_per_sm(bool reflect, bool savedet, int mode, int block, siz
 // (cyclic cube, 3e5: 10.6 with 2 CTAs, 8.7 with 3).
 // Where even that leaves every warp of the full grid no more than four photons, the full grid: 1e4 photons, a warp's
 // spread over its lanes as below, 1.35 / 1.30 / 1.23 on the cube, 1.54 / 1.51 / 1.49 with detectors (3e4: 1.49 / 1.53 / 1.68).
-int transport_grid(const KParams& p, int grid, int block, int sms, unsigned long long n) {
+int transport_grid(const KParams& p, bool savedet, int grid, int block, int sms, unsigned long long n) {
     for (int i = 0; i < 6; i++)
         if (p.bc[i] == BC_MIRROR || p.bc[i] == BC_CYCLIC) return grid;
-    if (transport_mode(p) >= kLeanPencil && n <= 4ull * (unsigned)grid * (unsigned)(block / 32)) return grid;
+    if (transport_mode(p, savedet) >= kLeanPencil && n <= 4ull * (unsigned)grid * (unsigned)(block / 32)) return grid;
     const unsigned long long a_round = 4ull * (unsigned)block * (unsigned)sms;
     const unsigned long long rounds = (n + a_round - 1) / a_round;
     return (unsigned long long)grid <= rounds * (unsigned)sms ? grid : (int)(std::max(rounds, 1ull) * (unsigned)sms);
@@ -1788,7 +1790,7 @@ cudaError_t launch_transport(const KParams& in, bool reflect, bool savedet, int 
     p.ahead = p.chunk > 1 ? 32u : 4u;
     // the caller sized the shared memory for the variant of its parameters: never launch another's
     if (smem_bytes < transport_smem_bytes(p, block, savedet)) return cudaErrorInvalidValue;
-    const void* k = pick(reflect, savedet, transport_mode(p), few);
+    const void* k = pick(reflect, savedet, transport_mode(p, savedet), few);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
     if (e != cudaSuccess) return e;
     void* args[] = {const_cast<KParams*>(&p)};

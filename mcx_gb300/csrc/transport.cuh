@@ -209,12 +209,12 @@ size_t transport_smem_bytes(const KParams& p, int block, bool savedet);
 // 3 = everything of 2 on a per-voxel media format, 4 = split voxels; kLeanPencil / kLeanArea = 0 / 1
 // on the plain path (transport_lean.cuh), kLeanReplay = its replay into the absorption Jacobians.
 constexpr int kLeanPencil = 8, kLeanArea = 9, kLeanReplay = 10;
-int transport_mode(const KParams& p);
-bool transport_general(const KParams& p);
+constexpr size_t kSmemPerCta = 227 * 1024;      // shared memory a CTA may have (sm_103a)
+int transport_mode(const KParams& p, bool savedet);
 // Occupancy-derived CTAs per SM for the chosen variant.
 int transport_blocks_per_sm(bool reflect, bool savedet, int mode, int block, size_t smem_bytes);
 // CTAs to launch for n photons on their own streams, at most `grid` (whole CTAs on every one of `sms` SMs).
-int transport_grid(const KParams& p, int grid, int block, int sms, unsigned long long n);
+int transport_grid(const KParams& p, bool savedet, int grid, int block, int sms, unsigned long long n);
 // Lanes of a warp left without a photon in a run of n (KParams::spare), for a launch that has the GPU to itself.
 unsigned transport_spare(int grid, int block, unsigned long long n);
 

@@ -52,10 +52,10 @@ struct LeanSmem {
     float ppath[1];                             // partialdata x kLeanBlock (detector runs), then the tile
 };
 
-inline size_t lean_smem_bytes(const KParams& p, bool savedet) {
+inline size_t lean_smem_bytes(const KParams& p, bool savedet, bool tile) {
     size_t b = offsetof(LeanSmem, ppath);
     if (savedet) b += sizeof(float) * (size_t)p.partialdata * kLeanBlock;
-    if (p.tile_on) b += sizeof(unsigned) * (size_t)p.tnx * p.tny * p.tnz * p.tng;
+    if (tile) b += sizeof(unsigned) * (size_t)p.tnx * p.tny * p.tnz * p.tng;
     return b;
 }
 
