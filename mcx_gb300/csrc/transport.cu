@@ -1149,7 +1149,8 @@ __global__ void __launch_bounds__(256, MINB) transport_kernel(const __grid_const
         t = fmaf(len, pr.w, t);                                         // t += len*n/c0, in grid units
         pathlen += len;
         // step cap, checked every 1024 steps of the lane against its step count at launch
-        if ((c_step & 1023u) == 0u && c_step - S.step0[tid] >= P.step_cap) {
+        const auto capped = [&] { return (c_step & 1023u) == 0u && c_step - S.step0[tid] >= P.step_cap; };
+        if (capped()) {
             atomicOr(P.errflag, kErrStepCap);
             kill = true;
         }
@@ -1296,7 +1297,9 @@ __global__ void __launch_bounds__(256, MINB) transport_kernel(const __grid_const
         }
         if (t > tw1) kill = true;
 
-        if (kill && !inside && bcf == BC_CYCLIC) {                      // 2311-2335
+        // (never for the step cap: on a periodic axis one voxel thick every step ends here)
+        // (asked again rather than kept: the value kept past the branches cost every step 1%)
+        if (kill && !inside && bcf == BC_CYCLIC && !capped()) {         // 2311-2335
             const float span = (axis == 0) ? fnx : ((axis == 1) ? fny : fnz);
             const float shift = (idx == kOUT_MIN) ? span : -span;
             if (axis == 0) { px = nextafter_mcx(roundf(px + shift), (vx > 0.f) - (vx < 0.f), P.maxvoidstep); fx = floorf(px); }

@@ -475,7 +475,8 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
                 kill = true;
         }
         bool wrapped = false;
-        if (kill && !valid && bcf == BC_CYCLIC) {                       // 2311-2335
+        // (never for the step cap: on a periodic axis one voxel thick every step ends here)
+        if (kill && left != 0u && !valid && bcf == BC_CYCLIC) {         // 2311-2335
             const float span = (axis == 0) ? P.d_fnx : ((axis == 1) ? P.d_fny : P.d_fnz);
             const float shift = outmax ? -span : span;
             if (axis == 0) { px = nextafter_mcx(roundf(px + shift), (vx > 0.f) - (vx < 0.f), P.maxvoidstep); fx = floorf(px); }
