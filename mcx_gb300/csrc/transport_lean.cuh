@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
                         const unsigned take = max(cnt, P.ahead);
                         unsigned long long base = 0ull;
                         if (lane == 0) base = atomicAdd(P.work, (unsigned long long)take);
-                        base = __shfl_sync(kFull, base, 0);     // and every lane has read the entries before
+                        base = __shfl_sync(kFull, base, 0);
+                        __syncwarp();           // every lane has read the entries before that are overwritten here
                         if (lane < take && base + lane < P.d_nwork) {
                             ulonglong2 q;
                             seed_photon(P.seed, P.photon_offset + base + lane, q.x, q.y);
@@ -211,7 +212,7 @@ __global__ void __launch_bounds__(kLeanBlock, MINB) lean_kernel(const __grid_con
                         q_next = tid - lane;
                         q_left = base >= P.d_nwork ? 0u : (unsigned)min((unsigned long long)take, P.d_nwork - base);
                         if (q_left == 0u) refill_at = kNever;
-                        __syncwarp();
+                        __syncwarp();           // and reads the new ones after they are written
                     }
                     start = !alive && rank < q_left;
                     if (start) {
