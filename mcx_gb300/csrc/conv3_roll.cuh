@@ -164,10 +164,17 @@ struct RollRing {
     }
 };
 
-// 16 consecutive bf16 outputs of a voxel: bias, ReLU, the mask, and one 32-byte store (two of 16 where the tensors
-// are aligned to 16 bytes only).
-__device__ __forceinline__ void roll_store16(const uint32_t* v, const float* bias, const bf16* __restrict__ mask,
-                                             bf16* __restrict__ y, int relu, bool wide) {
+// 16 channels of the mask.  An ordinary load, and no kernel that is launched chained declares the mask or the bias
+// __restrict__: the kernel ahead may write them after this one has started (chain_wait), so they are not read-only for its
+// lifetime, as the read-only path needs.
+__device__ __forceinline__ void roll_mask16(const bf16* mask, uint32_t* mk) {
+    *reinterpret_cast<uint4*>(mk) = *reinterpret_cast<const uint4*>(mask);
+    *reinterpret_cast<uint4*>(mk + 4) = *(reinterpret_cast<const uint4*>(mask) + 1);
+}
+
+// 16 consecutive bf16 outputs of a voxel: bias, ReLU, the mask's 16 values (or null), and one 32-byte store (two of 16
+// where the tensors are aligned to 16 bytes only).
+__device__ __forceinline__ void roll_store16(const uint32_t* v, const float* bias, const uint32_t* mk, bf16* y, int relu, bool wide) {
     uint32_t pk[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
@@ -179,10 +186,7 @@ __device__ __forceinline__ void roll_store16(const uint32_t* v, const float* bia
         __nv_bfloat162 h2 = __floats2bfloat162_rn(a, b);
         pk[e] = *reinterpret_cast<uint32_t*>(&h2);
     }
-    if (mask) {
-        uint32_t mk[8];
-        *reinterpret_cast<uint4*>(mk) = __ldg(reinterpret_cast<const uint4*>(mask));
-        *reinterpret_cast<uint4*>(mk + 4) = __ldg(reinterpret_cast<const uint4*>(mask) + 1);
+    if (mk) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             // keep each bf16 where the mask's bf16 is > 0 (sign bit clear and not +0)
@@ -203,8 +207,7 @@ __device__ __forceinline__ void roll_store16(const uint32_t* v, const float* bia
 template <int BN, bool TAPS>
 __global__ void __launch_bounds__(320, 1) conv3_roll_kernel(const __grid_constant__ CUtensorMap xmap,
                                                             const __grid_constant__ CUtensorMap wmap,
-                                                            const float* __restrict__ bias, const bf16* __restrict__ mask,
-                                                            bf16* __restrict__ y, Geo g, int cin, int cout, int relu, int tiles_x,
+                                                            const float* bias, const bf16* mask, bf16* y, Geo g, int cin, int cout, int relu, int tiles_x,
                                                             int tiles_y, int planes, int chunk, int stages, int wbufs, int wide) {
     using S = RollShape<BN>;
     constexpr int R = S::R, RP = S::RP;
@@ -476,7 +479,7 @@ __global__ void __launch_bounds__(320, 1) conv3_roll_kernel(const __grid_constan
         float bs[BN];
         while (!fault && run.next()) {
 #pragma unroll
-            for (int c = 0; c < BN; ++c) bs[c] = bias ? __ldg(bias + run.n0 + c) : 0.f;
+            for (int c = 0; c < BN; ++c) bs[c] = bias ? bias[run.n0 + c] : 0.f;
             const int yy = run.y0 + (r >> 3), xx = run.x0 + (r & 7);
             const bool in = yy < g.h && xx < g.w;
             const long long hw = (long long)g.h * g.w;
@@ -504,9 +507,19 @@ __global__ void __launch_bounds__(320, 1) conv3_roll_kernel(const __grid_constan
                     }
                     if (in && o + zz < run.nz) {
                         const long long at = (v0 + (o + zz) * hw) * cout + run.n0;
+                        // the mask of up to 48 channels before their first store, which it must not wait for
+                        constexpr int MB = BN > 48 ? BN / 2 : BN;
 #pragma unroll
-                        for (int c0 = 0; c0 < BN; c0 += 16)
-                            roll_store16(v + c0, bs + c0, mask ? mask + at + c0 : nullptr, y + at + c0, relu, wide != 0);
+                        for (int b = 0; b < BN; b += MB) {
+                            uint32_t mk[MB / 2];
+                            if (mask) {
+#pragma unroll
+                                for (int c0 = 0; c0 < MB; c0 += 16) roll_mask16(mask + at + b + c0, mk + c0 / 2);
+                            }
+#pragma unroll
+                            for (int c0 = 0; c0 < MB; c0 += 16)
+                                roll_store16(v + b + c0, bs + b + c0, mask ? mk + c0 / 2 : nullptr, y + at + b + c0, relu, wide != 0);
+                        }
                     }
                 }
             }

@@ -53,8 +53,7 @@ struct StreamTile {
 
 __global__ void __launch_bounds__(224, 1) conv3_stream_kernel(const __grid_constant__ CUtensorMap xmap,
                                                               const __grid_constant__ CUtensorMap wmap,
-                                                              const float* __restrict__ bias, const bf16* __restrict__ mask,
-                                                              bf16* __restrict__ y, Geo g, int cin, int cout, int relu, int tiles_x,
+                                                              const float* bias, const bf16* mask, bf16* y, Geo g, int cin, int cout, int relu, int tiles_x,
                                                               int tiles_y, int tiles, int wbufs, int wide) {
     using S = StreamShape;
     constexpr int BN = S::BN;
@@ -193,10 +192,15 @@ __global__ void __launch_bounds__(224, 1) conv3_stream_kernel(const __grid_const
                 const long long at = ((((long long)tile.n * g.d + tile.z) * g.h + yy) * g.w + xx) * cout + tile.n0;
                 float bs[BN];
 #pragma unroll
-                for (int c = 0; c < BN; ++c) bs[c] = bias ? __ldg(bias + tile.n0 + c) : 0.f;
+                for (int c = 0; c < BN; ++c) bs[c] = bias ? bias[tile.n0 + c] : 0.f;
+                uint32_t mk[BN / 2];
+                if (mask) {
+#pragma unroll
+                    for (int c0 = 0; c0 < BN; c0 += 16) roll_mask16(mask + at + c0, mk + c0 / 2);
+                }
 #pragma unroll
                 for (int c0 = 0; c0 < BN; c0 += 16)
-                    roll_store16(v + c0, bs + c0, mask ? mask + at + c0 : nullptr, y + at + c0, relu, wide != 0);
+                    roll_store16(v + c0, bs + c0, mask ? mk + c0 / 2 : nullptr, y + at + c0, relu, wide != 0);
             }
         }
     }
