@@ -42,15 +42,31 @@ __device__ __forceinline__ uint64_t umma_desc_mn32(uint32_t saddr, uint32_t lbo,
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (6ull << 61);
 }
 
-// The sums of a CTA's group over its run, voxel by voxel: for a run that holds an infinity or a NaN (below).
+// A CTA's group over its run on mma.sync, without the products of voxels outside the volume: for a run whose sums hold an
+// infinity or a NaN (below).  The same tiles, copied to shared memory by all threads; a row of X that a voxel of dY outside
+// the volume would meet is read as zeros.  A warp holds 16 output channels x three pairs x three dz; where there
+// are fewer such units than warps, they share a unit's K steps.  Bound by the copies, which nothing overlaps.  Rare, but a
+// training step that meets one infinity should not stall (GB300, us a call: finite, one infinity, X all NaN, and the
+// general kernel on any of them): 2 x 65^3 16 to 16 41, 197, 209, 113; 4 x 65^3 48 to 16 180, 913, 1180, 636; 4 x 33^3
+// 96 to 32 85, 722, 790, 176; 33^3 64 to 64 32, 198, 241, 49; 4 x 17^3 128 to 128 66, 960, 992, 76.  (A voxel at a time on the
+// CUDA cores took 7.7 to 38 ms for one infinity and 14 to 110 for X all NaN.)
 template <int COUT>
-__device__ __noinline__ void wgrad_by_voxel(const bf16* dy, const bf16* x, float* dw, const Geo& g, int cin, int tiles_x, int tiles_y,
-                                            int tiles_z, int t_lo, int t_hi, int pair0, int pairs) {
-    constexpr int PZ = WgradShape<COUT>::PZ;
-    for (int o = threadIdx.x; o < pairs * 3 * COUT * 16; o += blockDim.x) {
-        const int ci = o % 16, co = o / 16 % COUT, dz = o / (16 * COUT) % 3, pair = pair0 + o / (48 * COUT);
-        const int tap = pair % 9, cx = pair / 9 * 16 + ci;
-        float sum = 0.f;
+__device__ __noinline__ void wgrad_within(unsigned char* smem, const bf16* dy, const bf16* x, float* dw, const Geo& g, int cin, int tiles_x,
+                                          int tiles_y, int tiles_z, int t_lo, int t_hi, int pair0, int pairs) {
+    using S = WgradShape<COUT>;
+    constexpr int PZ = S::PZ, WARPS = 6;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int slice0 = pair0 / 9, nsl = (pair0 + pairs - 1) / 9 - slice0 + 1;
+    const int xchunks = nsl * (PZ + 2) * 180 * 2;
+    uint4* const sy = reinterpret_cast<uint4*>(smem);               // [Cout / 16][PZ][16][8] rows of 32 bytes
+    uint4* const sx = sy + S::YBYTES / 16;                          // [nsl][PZ + 2][18][10] rows
+    uint4* const zeros = sx + xchunks;                              // a row
+    const int trios = (pairs + 2) / 3, units = COUT / 16 * trios, share = units < WARPS ? WARPS / units : 1;
+    for (int base = 0; base < units * share; base += WARPS) {
+        const int unit = (base + warp) / share, part = (base + warp) % share;
+        const bool on = unit < units;
+        const int mb = unit / trios, p0 = unit % trios * 3;
+        float acc[3][3][2][4] = {};
         for (int t = t_lo; t < t_hi; ++t) {
             int r = t;
             const int x0 = (r % tiles_x) * 8;
@@ -58,20 +74,58 @@ __device__ __noinline__ void wgrad_by_voxel(const bf16* dy, const bf16* x, float
             const int y0 = (r % tiles_y) * 16;
             r /= tiles_y;
             const int z0 = (r % tiles_z) * PZ, n = r / tiles_z;
-            float s = 0.f;
-            for (int z = z0; z < min(z0 + PZ, g.d); ++z)
-                for (int y = y0; y < min(y0 + 16, g.h); ++y)
-                    for (int xx = x0; xx < min(x0 + 8, g.w); ++xx) {
-                        const int uz = z + dz - 1, uy = y + tap / 3 - 1, ux = xx + tap % 3 - 1;
-                        const bool in = (unsigned)uz < (unsigned)g.d && (unsigned)uy < (unsigned)g.h && (unsigned)ux < (unsigned)g.w;
-                        const float a = __bfloat162float(dy[(((long long)n * g.d + z) * g.h + y) * g.w * COUT + (long long)xx * COUT + co]);
-                        const float b =
-                            in ? __bfloat162float(x[((((long long)n * g.d + uz) * g.h + uy) * g.w + ux) * cin + cx]) : 0.f;
-                        s = fmaf(a, b, s);
+            const auto voxel = [&](int z, int y, int xx) { return (((long long)n * g.d + z) * g.h + y) * g.w + xx; };
+            const auto within = [&](int z, int y, int xx) {
+                return (unsigned)z < (unsigned)g.d && (unsigned)y < (unsigned)g.h && (unsigned)xx < (unsigned)g.w;
+            };
+            __syncthreads();        // the tile before has been read
+            for (int i = tid; i < S::YBYTES / 16; i += 32 * WARPS) {
+                const int xx = x0 + (i >> 1) % 8, yy = y0 + (i >> 4) % 16, zz = z0 + (i >> 8) % PZ, c = (i >> 8) / PZ * 16 + (i & 1) * 8;
+                const bool in = within(zz, yy, xx);
+                cp_async16(smem_addr(sy + i), in ? dy + voxel(zz, yy, xx) * COUT + c : dy, in);
+            }
+            for (int i = tid; i < xchunks; i += 32 * WARPS) {
+                const int v = i >> 1, s = v / (180 * (PZ + 2)), c = (slice0 + s) * 16 + (i & 1) * 8;
+                const int xx = x0 - 1 + v % 10, yy = y0 - 1 + v / 10 % 18, zz = z0 - 1 + v / 180 % (PZ + 2);
+                const bool in = within(zz, yy, xx);
+                cp_async16(smem_addr(sx + i), in ? x + voxel(zz, yy, xx) * cin + c : x, in);
+            }
+            if (tid < 2) zeros[tid] = make_uint4(0u, 0u, 0u, 0u);
+            cp_commit();
+            cp_wait<0>();
+            __syncthreads();
+            for (int k = part; on && k < PZ * 8; k += share) {      // a K step: two y rows of 8 voxels
+                const int p = k >> 3, y = (k & 7) * 2, m = lane >> 3, xx = lane & 7;
+                if (z0 + p >= g.d) break;
+                uint32_t a[4], b[4];
+                ldsm_x4_t(smem_addr(sy + (((mb * PZ + p) * 16 + y + (m >> 1)) * 8 + xx) * 2 + (m & 1)), a);
+                const bool in = within(z0 + p, y0 + y + (m & 1), x0 + xx);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const int pair = pair0 + p0 + i, tap = pair % 9;
+                    if (p0 + i >= pairs) break;
+#pragma unroll
+                    for (int dz = 0; dz < 3; ++dz) {
+                        const int row = (((pair / 9 - slice0) * (PZ + 2) + p + dz) * 18 + y + (m & 1) + tap / 3) * 10 + xx + tap % 3;
+                        ldsm_x4_t(smem_addr((in ? sx + row * 2 : zeros) + (m >> 1)), b);
+                        mma_bf16(acc[i][dz][0], a, b[0], b[1]);
+                        mma_bf16(acc[i][dz][1], a, b[2], b[3]);
                     }
-            sum += s;
+                }
+            }
         }
-        atomicAdd(dw + ((long long)co * 27 + dz * 9 + tap) * cin + cx, sum);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int pair = pair0 + p0 + i;
+            if (!on || p0 + i >= pairs) break;
+#pragma unroll
+            for (int dz = 0; dz < 3; ++dz)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const int co = mb * 16 + (lane >> 2) + (e >> 1 & 1) * 8, ci = pair / 9 * 16 + (e >> 2) * 8 + (lane & 3) * 2 + (e & 1);
+                    atomicAdd(dw + ((long long)co * 27 + dz * 9 + pair % 9) * cin + ci, acc[i][dz][e >> 2][e & 3]);
+                }
+        }
     }
 }
 
@@ -200,7 +254,7 @@ __global__ void __launch_bounds__(192, 1) conv3_wgrad_kernel(const __grid_consta
             }
         }
         plain = __syncthreads_or(odd) == 0;
-        if (!plain) wgrad_by_voxel<COUT>(dy, x, dw, g, cin, tiles_x, tiles_y, tiles_z, t_lo, t_hi, pair0, pairs);
+        if (!plain) wgrad_within<COUT>(dyn_smem, dy, x, dw, g, cin, tiles_x, tiles_y, tiles_z, t_lo, t_hi, pair0, pairs);
     }
     if (warp < 4 && ok && plain) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
