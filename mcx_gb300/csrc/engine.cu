@@ -409,6 +409,7 @@ struct Session {
     int block = 256, grid = 0, sms = 0;
     int run_grid = 0;          // CTAs of the last launch: `grid` or fewer for a run of few photons
     bool fixed_grid = false;   // CTAs per SM given by mcxg_set_launch
+    bool alone = true;         // no other session of the same run on this device
     size_t smem = 0;
     size_t nvox = 0, fieldlen = 0;
     int totalgates = 1;
@@ -823,6 +824,11 @@ struct Session {
         kp.twin1 = twin1;
     }
 
+    // CTAs of a launch over n photons that `run` makes.
+    int grid_for(uint64_t n) const {
+        return (kp.seed_mode == 1 || fixed_grid) ? grid : transport_grid(kp, savedet, grid, block, sms, n);
+    }
+
     // One persistent transport launch over photons [offset, offset + n).
     // `beside`, when given, runs on the host while the GPU works.
     template <class F>
@@ -837,8 +843,8 @@ struct Session {
             kp.mcx_odd = (unsigned)(n - (uint64_t)kp.mcx_per * mcx_streams);
         }
         CK(cudaMemsetAsync(work.p, 0, sizeof(unsigned long long), stream));
-        run_grid = (kp.seed_mode == 1 || fixed_grid) ? grid : transport_grid(kp, savedet, grid, block, sms, n);
-        kp.spare = transport_spare(run_grid, block, n);
+        run_grid = grid_for(n);
+        kp.spare = alone ? transport_spare(run_grid, block, n) : 0;
         CK(cudaEventRecord(ev0, stream));
         CK(launch_transport(kp, reflect, savedet, run_grid, block, smem, stream));
         CK(cudaEventRecord(ev1, stream));
@@ -1507,6 +1513,7 @@ void run_simulation(Config* cfg, GPUInfo* gpu, bool fp64_field) {
             SS[d]->create(cfg, ids[d], fp64_field, maxgate);
         }
     });
+    for (int d = 0; d < ndev; d++) SS[d]->alone = std::count(ids.begin(), ids.end(), ids[d]) == 1;
     Session& S = *SS[0];
     {
         // large runs tune the deposit tile with short pilot launches (cached per configuration)
@@ -1529,7 +1536,7 @@ void run_simulation(Config* cfg, GPUInfo* gpu, bool fp64_field) {
     if (cfg->flog && cfg->printnum >= 0)
         for (int d = 0; d < ndev; d++)
             fprintf(cfg->flog, "GPU=%d (%s) np=%.0f grid=%d block=%d chunk=%d maxgate=%d repetition=%d\n", ids[d] + 1,
-                    gpu ? gpu[ids[d]].name : "", (double)count[d] * (cfg->respin > 0 ? 1 : reps), SS[d]->grid,
+                    gpu ? gpu[ids[d]].name : "", (double)count[d] * (cfg->respin > 0 ? 1 : reps), SS[d]->grid_for(count[d]),
                     SS[d]->block, SS[d]->kp.chunk, maxgate, reps);
 
     std::vector<float> host_field;
@@ -1567,7 +1574,7 @@ void run_simulation(Config* cfg, GPUInfo* gpu, bool fp64_field) {
     int threads = 0;
     for (auto& p : SS) {
         kernel_ms = std::max(kernel_ms, p->kernel_ms);
-        threads += p->grid * p->block;
+        threads += p->run_grid * p->block;
     }
     total.kernel_ms = kernel_ms;
     total.total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
