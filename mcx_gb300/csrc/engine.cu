@@ -30,7 +30,7 @@
 #include <mutex>
 #include <stdlib.h>
 #include <string>
-#include <system_error>
+#include <exception>
 #include <unistd.h>
 #include <thread>
 #include <vector>
@@ -141,7 +141,7 @@ public:
         size_t t = 0;
         try {
             for (; t + 1 < nt; t++) th_.emplace_back(touch, pages * t / nt, pages * (t + 1) / nt);
-        } catch (const std::system_error&) {        // no thread to be had: the caller does what is left
+        } catch (const std::exception&) {           // no thread or no memory for one: the caller does what is left
         }
         touch(nt > 1 ? pages * t / nt : 0, pages);
     }

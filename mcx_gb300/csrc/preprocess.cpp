@@ -21,7 +21,7 @@
 #include <ctime>
 #include <algorithm>
 #include <mutex>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -322,11 +322,11 @@ void in_parallel(size_t n, size_t least, F&& f) {
         return;
     }
     std::vector<std::thread> th;
-    th.reserve(nt);
     size_t t = 0;
     try {
+        th.reserve(nt);
         for (; t + 1 < nt; t++) th.emplace_back(f, n * t / nt, n * (t + 1) / nt);
-    } catch (const std::system_error&) {        // no thread to be had: the caller does what is left
+    } catch (const std::exception&) {           // no thread or no memory for one: the caller does what is left
     }
     f(n * t / nt, n);
     for (auto& x : th) x.join();
