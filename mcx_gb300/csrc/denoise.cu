@@ -1156,7 +1156,8 @@ void allow_smem(K kern, int dev, std::atomic<unsigned long long>& done) {
         done.fetch_or(bit, std::memory_order_relaxed);
 }
 
-// Launch of conv3_roll_kernel for BN output channels a block (BN divides cout).
+// Launch of conv3_roll_kernel for BN output channels a block (BN divides cout).  Returns 1 where its planes are too many to
+// count in 32 bits (volumes of a voxel a plane, many channel blocks): the general kernels count voxels.
 template <int BN, bool TAPS>
 int conv3_roll_launch(const bf16* x, const bf16* w, const float* bias, const bf16* mask, bf16* y, Geo g, int cin,
                       int cout, int relu, int dev, int sms, cudaStream_t st) {
@@ -1190,7 +1191,7 @@ int conv3_roll_launch(const bf16* x, const bf16* w, const float* bias, const bf1
     }
     const int tx = (g.w + S::TX - 1) / S::TX, ty = (g.h + S::TY - 1) / S::TY;
     const long long planes = (long long)(cout / BN) * g.nvol * tx * ty * g.d;
-    if (planes >= (1LL << 31)) return fail("conv: too many tiles");
+    if (planes >= (1LL << 31)) return 1;
     const int slices = cin / 16, stage = TAPS ? slices * S::ENTRY : S::STAGE;
     // all slices' weights beside the halo stages (tap-major: always; else beside at least four, or a ring of two)
     int wbufs = slices;
@@ -1232,7 +1233,7 @@ double roll_cost(const Geo& g, int cin, int cout, int bn, bool taps, int sms) {
     return math > copies ? math : copies;
 }
 
-// `taps`: the tap-major order.  Returns 1 where no block width fits it.
+// `taps`: the tap-major order.  Returns 1 where no block width fits it, or the launch does not take it.
 int conv3_roll_dispatch(const bf16* x, const bf16* w, const float* bias, const bf16* mask, bf16* y, Geo g, int cin,
                         int cout, int relu, bool taps, cudaStream_t st) {
     int dev = 0, sms = 0;
