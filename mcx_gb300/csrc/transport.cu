@@ -1707,6 +1707,10 @@ int transport_blocks_per_sm(bool reflect, bool savedet, int mode, int block, siz
 // 256^3, 1e5 11.9 / 12.6 / 14.2 and 1e6 35.9 / 26.5 / 25.9.
 // Not where a face mirrors photons or hands them to the other side: they all live as long, and the fuller SM wins
 // (cyclic cube, 3e5: 10.6 with 2 CTAs, 8.7 with 3).
+// The general kernel likewise (ms, full grid / this rule): reflecting cube at 1e4, 1e5, 3e5 photons 3.83 / 3.67, 5.64 / 4.13,
+// 6.51 / 5.10; with seeds saved 5.36 / 5.36, 9.70 / 6.08, 12.2 / 9.6; planar source 3.89 / 3.57, 4.82 / 4.06, 5.69 / 5.24;
+// layered head 128^3 28.9 / 29.0, 34.2 / 33.2, 44.3 / 38.0, with roulette 8.41 / 8.56, 10.3 / 9.4, 13.0 / 12.2; media by
+// voxel 8.43 / 8.36, 11.7 / 10.6, 13.7 / 13.2; a replay into flux of 6763 and 22470 photons 4.96 / 4.93, 4.94 / 4.92.
 // Where even that leaves every warp of the full grid no more than four photons, the full grid: 1e4 photons, a warp's
 // spread over its lanes as below, 1.35 / 1.30 / 1.23 on the cube, 1.54 / 1.51 / 1.49 with detectors (3e4: 1.49 / 1.53 / 1.68).
 int transport_grid(const KParams& p, bool savedet, int grid, int block, int sms, unsigned long long n) {
