@@ -14,7 +14,9 @@
 // An accumulator per (slice of 16 input channels, dydx tap), N columns each: tensor memory holds G = 512 / N of them, a
 // group.  A CTA takes one group over a run of tiles (16 y x 8 x x PZ z), two or more tiles in flight, and at the end adds
 // the diagonals of its accumulators over the planes, through shared memory over its warps, to dW with vector
-// reductions.  A sum in tensor memory is as long as the run, at most a few hundred K steps.
+// reductions.  A sum in tensor memory is as long as the run, eight K steps a tile: 88 at 2 x 64^3 16 to 16, 4096 at 4 x
+// 128^3 48 to 16, about a fifth of the general kernel's chains (there, on operands with a mean, it is off by 3.0e-5 of the sum of
+// absolute values, the general kernel by 1.5e-4).
 //
 // Roles: warp 4 issues the copies, warp 5 the MMAs (converged, one elected lane), warps 0-3 the epilogue.  Every wait is
 // bounded and reports through g_dn_fault.

@@ -523,11 +523,7 @@ void validate(Config* cfg) {
 
 }  // namespace
 
-// mcx_replayinit (src/mcx_utils.c:3624-3690): keep the detected photons of detector `replaydet`
-// (all when <= 0) whose time of flight lies in [tstart, tend], with their seeds, detected weight
-// exp(-sum mua_m ppath_m), time of flight sum ppath_m n_m / c0 and detector id.  detps holds
-// dimdetps[1] records of dimdetps[0] floats (savedetflag with D and P); seeds arrive in
-// cfg->replay.seed, seedbyte bytes per photon, and are compacted in place.  Sets nphoton.
+// Integer labels in C order to 32 bits in x-fastest order (contract in include/mcx_gb300.h).
 extern "C" int mcxg_widen_labels(const void* src, int itemsize, int is_signed, unsigned nx, unsigned ny, unsigned nz,
                                  uint32_t* dst) {
     if (!src || !dst || !nx || !ny || !nz) return -4;
@@ -545,6 +541,11 @@ extern "C" int mcxg_widen_labels(const void* src, int itemsize, int is_signed, u
     }
 }
 
+// mcx_replayinit (src/mcx_utils.c:3624-3690): keep the detected photons of detector `replaydet`
+// (all when <= 0) whose time of flight lies in [tstart, tend], with their seeds, detected weight
+// exp(-sum mua_m ppath_m), time of flight sum ppath_m n_m / c0 and detector id.  detps holds
+// dimdetps[1] records of dimdetps[0] floats (savedetflag with D and P); seeds arrive in
+// cfg->replay.seed, seedbyte bytes per photon, and are compacted in place.  Sets nphoton.
 extern "C" int mcxg_replayinit(Config* cfg, const float* detps, const int dimdetps[2], int seedbyte) {
     mcxg_clear_error();
     try {
