@@ -397,6 +397,33 @@ void fill_source(KParams& k, const Config* cfg, const float* d_pattern) {
     }
 }
 
+// Photons a thread that transport_grid leaves a run of few photons: four where the photons come in through the face of a
+// volume ten transport lengths thick or more, so that most soon leave again and a few live ten times as long as the mean;
+// one where they live alike: started inside, or crossing a thin or nearly clear volume.  (Of media by voxel the first row
+// of the table stands for the rest.)
+unsigned photons_a_thread(const Config* cfg, const KParams& k) {
+    switch (k.srctype) {        // beams; the other sources send photons every way or fill a volume
+        case kSrcPencil: case kSrcGaussian: case kSrcPlanar: case kSrcPattern: case kSrcFourier: case kSrcDisk: case kSrcFourierX:
+        case kSrcFourierX2D: case kSrcPencilArray: case kSrcHyperboloid: case kSrcRing: break;
+        default: return 1;
+    }
+    if (k.src_focus != kFocusNone || cfg->nangle || cfg->extrasrclen) return 1;
+    const float4 p = cfg->srcpos, v = cfg->srcdir;
+    const auto label = [&](float s) -> uint32_t {       // s voxels along the beam; 0 outside
+        const float x = std::floor(p.x + s * v.x), y = std::floor(p.y + s * v.y), z = std::floor(p.z + s * v.z);
+        if (!(x >= 0.f && y >= 0.f && z >= 0.f && x < (float)k.nx && y < (float)k.ny && z < (float)k.nz)) return 0u;
+        const uint32_t w = host_label(cfg, (long)((unsigned)z * k.dimxy + (unsigned)y * (unsigned)k.nx + (unsigned)x));
+        return media_words(cfg->mediabyte) ? (w ? 1u : 0u) : w & kMED_MASK;
+    };
+    if (label(-1.f)) return 1;
+    uint32_t med = 0;
+    for (int s = 0; s <= k.nx + k.ny + k.nz + (int)k.maxvoidstep && !med; s++) med = label((float)s);
+    if (!med) med = 1;          // the beam's axis misses the volume: of a wide source only
+    if (med >= (uint32_t)k.medianum) return 1;
+    const float4 m = k.prop[med];
+    return m.y * (1.f - std::fabs(m.z)) * (float)std::min({k.nx, k.ny, k.nz}) >= 10.f ? 4u : 1u;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Session: one prepared simulation on one device.
 // ---------------------------------------------------------------------------------------------
@@ -409,6 +436,7 @@ struct Session {
     int block = 256, grid = 0, sms = 0;
     int run_grid = 0;          // CTAs of the last launch: `grid` or fewer for a run of few photons
     bool fixed_grid = false;   // CTAs per SM given by mcxg_set_launch
+    unsigned per_thread = 1;   // photons_a_thread
     bool alone = true;         // no other session of the same run on this device
     size_t smem = 0;
     size_t nvox = 0, fieldlen = 0;
@@ -565,6 +593,7 @@ struct Session {
             CK(cudaMemcpyAsync(pattern.p, cfg->srcpattern, npat * sizeof(float), cudaMemcpyHostToDevice, stream));
         }
         fill_source(k, cfg, pattern.as<float>());
+        per_thread = photons_a_thread(cfg, k);
         // user phase function and launch-angle tables (src/mcx_core.cu:1804-1836 stage them in
         // shared memory; here they are read through the read-only cache)
         k.nextra = (int)cfg->extrasrclen;
@@ -826,7 +855,7 @@ struct Session {
 
     // CTAs of a launch over n photons that `run` makes.
     int grid_for(uint64_t n) const {
-        return (kp.seed_mode == 1 || fixed_grid) ? grid : transport_grid(kp, savedet, grid, block, sms, n);
+        return (kp.seed_mode == 1 || fixed_grid) ? grid : transport_grid(kp, savedet, per_thread, grid, block, sms, n);
     }
 
     // One persistent transport launch over photons [offset, offset + n).

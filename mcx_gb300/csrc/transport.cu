@@ -1713,11 +1713,11 @@ int transport_blocks_per_sm(bool reflect, bool savedet, int mode, int block, siz
 // voxel 8.43 / 8.36, 11.7 / 10.6, 13.7 / 13.2; a replay into flux of 6763 and 22470 photons 4.96 / 4.93, 4.94 / 4.92.
 // Where even that leaves every warp of the full grid no more than four photons, the full grid: 1e4 photons, a warp's
 // spread over its lanes as below, 1.35 / 1.30 / 1.23 on the cube, 1.54 / 1.51 / 1.49 with detectors (3e4: 1.49 / 1.53 / 1.68).
-int transport_grid(const KParams& p, bool savedet, int grid, int block, int sms, unsigned long long n) {
+int transport_grid(const KParams& p, bool savedet, unsigned per_thread, int grid, int block, int sms, unsigned long long n) {
     for (int i = 0; i < 6; i++)
         if (p.bc[i] == BC_MIRROR || p.bc[i] == BC_CYCLIC) return grid;
     if (transport_mode(p, savedet) >= kLeanPencil && n <= 4ull * (unsigned)grid * (unsigned)(block / 32)) return grid;
-    const unsigned long long a_round = 4ull * (unsigned)block * (unsigned)sms;
+    const unsigned long long a_round = (unsigned long long)per_thread * (unsigned)block * (unsigned)sms;
     const unsigned long long rounds = (n + a_round - 1) / a_round;
     return (unsigned long long)grid <= rounds * (unsigned)sms ? grid : (int)(std::max(rounds, 1ull) * (unsigned)sms);
 }
