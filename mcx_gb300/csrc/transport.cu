@@ -736,6 +736,8 @@ __device__ __forceinline__ void flush_segment(const KParams& P, const Smem& S, i
     segp = 0.f;
 }
 
+constexpr float kNoTime = 3e38f;        // the time of a photon that the step cap has ended
+
 // MINB: CTAs of 256 threads the register budget is sized for (4 -> 64 registers, 3 -> 85, 2 -> 128).
 // MODE 0: pencil beam, flux / fluence / energy.  MODE 1: adds per-photon sampling of the other
 // source shapes.  MODE 2: adds replay, seed saving and the replay / path-length outputs.
@@ -1149,10 +1151,10 @@ __global__ void __launch_bounds__(256, MINB) transport_kernel(const __grid_const
         t = fmaf(len, pr.w, t);                                         // t += len*n/c0, in grid units
         pathlen += len;
         // step cap, checked every 1024 steps of the lane against its step count at launch
-        const auto capped = [&] { return (c_step & 1023u) == 0u && c_step - S.step0[tid] >= P.step_cap; };
-        if (capped()) {
+        if ((c_step & 1023u) == 0u && c_step - S.step0[tid] >= P.step_cap) {
             atomicOr(P.errflag, kErrStepCap);
             kill = true;
+            t = kNoTime;        // past every window: nothing may send the photon on
         }
 
         const unsigned detold = carry ? kDET_MASK : 0u;   // mediaidold's detector bit (src/mcx_core.cu:2167)
@@ -1297,9 +1299,9 @@ __global__ void __launch_bounds__(256, MINB) transport_kernel(const __grid_const
         }
         if (t > tw1) kill = true;
 
-        // (never for the step cap: on a periodic axis one voxel thick every step ends here)
-        // (asked again rather than kept: the value kept past the branches cost every step 1%)
-        if (kill && !inside && bcf == BC_CYCLIC && !capped()) {         // 2311-2335
+        // (never for the step cap: on a periodic axis one voxel thick every step ends here.  It shows in the time, which is
+        // kept anyway: a truth value kept past the branches cost every step 1%)
+        if (kill && !inside && bcf == BC_CYCLIC && !(t >= kNoTime)) {       // 2311-2335
             const float span = (axis == 0) ? fnx : ((axis == 1) ? fny : fnz);
             const float shift = (idx == kOUT_MIN) ? span : -span;
             if (axis == 0) { px = nextafter_mcx(roundf(px + shift), (vx > 0.f) - (vx < 0.f), P.maxvoidstep); fx = floorf(px); }
