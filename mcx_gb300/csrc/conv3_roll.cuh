@@ -465,8 +465,7 @@ __global__ void __launch_bounds__(320, 1) conv3_roll_kernel(const __grid_constan
                         done.step();
                     }
                 }
-                // (not after the last MMA: the epilogue waits for those, for this arrival nobody would before the CTA ends)
-                if (release && (after < run.end || sl + 1 < slices)) umma_commit(lead, wempty0 + 8 * wr.i);
+                if (release) umma_commit(lead, wempty0 + 8 * wr.i);
                 wr.step();
             }
             slot = done;
