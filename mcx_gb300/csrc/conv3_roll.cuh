@@ -470,6 +470,8 @@ __global__ void __launch_bounds__(320, 1) conv3_roll_kernel(const __grid_constan
             }
             slot = done;
         }
+        // the last release comes behind the commits that the epilogue waits for: it arrives before the CTA ends
+        if (!resident && !fault) fault = !warp_wait(wempty0 + 8 * ((wr.i == 0 ? wbufs : wr.i) - 1), wr.phase ^ (wr.i == 0 ? 1u : 0u));
     } else {
         // ---- epilogue: warps 0-3 and 4-7 take turns at pairs of planes ------------------------------------
         const int wg = warp >> 2, r = (warp & 3) * 32 + lane;       // accumulator row = TMEM lane = voxel of a plane
