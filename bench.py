@@ -52,13 +52,13 @@ CONTEST_DECKS = ("cube60", "cube60b", "cube60planar")
 
 # Thread-level instructions per transport step (ncu smsp__inst_executed.sum x
 # smsp__thread_inst_executed_per_inst_executed.ratio over the kernel's own step counter), one ncu
-# capture of lean_kernel per deck (8e6, 8e6 and 1e6 photons), and DRAM bytes of one launch
-# (dram__bytes_read.sum + dram__bytes_write.sum), from one ncu capture
-# of `bench.py --workload W --photons 20000000 --steps 1 --warmup 1` (workload2: 2000000).  The DRAM
-# bytes are the field's first read and its write-back: the field and labels stay in L2, so they do
+# capture of lean_kernel per deck (8e6, 8e6 and 1e6 photons), and DRAM bytes of one launch of it
+# (dram__bytes_read.sum + dram__bytes_write.sum), the last of an ncu capture
+# of `bench.py --workload W --photons 20000000 --steps 1 --warmup 1 --no-cpu-baseline` (workload2: 2000000).  The
+# DRAM bytes are the first read of the field and the labels: both stay in L2, so they do
 # not grow with the photon count.
 NCU_PER_STEP = {"workload0": 166.6, "workload1": 177.8, "workload2": 174.1}
-NCU_DRAM_PER_LAUNCH = {"workload0": 1.63e6, "workload1": 41.59e6, "workload2": 25.97e6}
+NCU_DRAM_PER_LAUNCH = {"workload0": 1.86e6, "workload1": 41.22e6, "workload2": 26.29e6}
 
 
 def _dist():

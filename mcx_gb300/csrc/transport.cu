@@ -1703,16 +1703,20 @@ int transport_blocks_per_sm(bool reflect, bool savedet, int mode, int block, siz
     return n;
 }
 
-// A run of few photons lasts as long as its longest one, step after step of one warp, and warps beside it on the
-// SM make its steps longer: fewer CTAs, so that a thread has about four photons, end sooner.  Measured (ms, 1 / 2 / 3
-// CTAs an SM): homogeneous cube, 1e5 photons 1.71 / 1.88 / 2.30; 3e5 2.26 / 2.22 / 2.70; 1e6 4.80 / 3.63 / 3.75; layered head
-// 256^3, 1e5 11.9 / 12.6 / 14.2 and 1e6 35.9 / 26.5 / 25.9.
+// A run of few photons lasts as long as its longest one, step after step of one warp, and warps beside it on the SM make
+// its steps longer: fewer CTAs, so that a thread has about `per_thread` photons, end sooner.  How many is the source's and the
+// volume's (photons_a_thread in engine.cu).  Measured (ms, 1 / 2 / 3 CTAs an SM):
+//   four where a beam enters a thick volume: cube, 1e5 photons 1.71 / 1.88 / 2.30, 3e5 2.26 / 2.22 / 2.70, 1e6 4.80 / 3.63 / 3.75;
+//   layered head 256^3, 1e5 11.9 / 12.6 / 14.2, 1e6 35.9 / 26.5 / 25.9; the general kernel on the cube, 1.5e5 3.09 / 3.17 / 3.60;
+//   one where photons live alike: isotropic source in the cube, 6e4 photons 3.03 / 2.53 / 3.20, 1e5 4.25 / 3.14 / 3.37, 1.5e5
+//   5.84 / 4.14 / 4.03; in 60^3 of mus 8, 14.9 / 9.4 / 12.2, 22.3 / 16.0 / 12.8, 29.9 / 18.4 / 17.3 (general kernel 23.4 / 13.6 / 15.8,
+//   33.8 / 25.3 / 17.0, 44.6 / 27.3 / 27.2); a beam through 24^3 of mus 0.3, 1.5e5 0.39 / 0.34 / 0.35.
+// The general kernel with this rule against its full grid (ms, at 1e5 and 3e5 photons): reflecting cube 5.64 / 4.13, 6.51 / 5.10;
+// with seeds saved 9.70 / 6.06, 12.2 / 9.5; planar source 4.82 / 4.06, 5.69 / 5.24; layered head 128^3 34.2 / 33.5, 44.3 / 37.8,
+// with roulette 10.3 / 9.7, 13.0 / 12.4; media by voxel 11.7 / 10.3, 13.7 / 12.8; split voxels 14.9 / 14.0, 19.6 / 17.8;
+// trajectories 6.89 / 5.89, 9.09 / 7.27; polarised light through a thin slab 1.30 / 1.30, 2.13 / 2.06.  At 1e4 the same.
 // Not where a face mirrors photons or hands them to the other side: they all live as long, and the fuller SM wins
 // (cyclic cube, 3e5: 10.6 with 2 CTAs, 8.7 with 3).
-// The general kernel likewise (ms, full grid / this rule): reflecting cube at 1e4, 1e5, 3e5 photons 3.83 / 3.67, 5.64 / 4.13,
-// 6.51 / 5.10; with seeds saved 5.36 / 5.36, 9.70 / 6.08, 12.2 / 9.6; planar source 3.89 / 3.57, 4.82 / 4.06, 5.69 / 5.24;
-// layered head 128^3 28.9 / 29.0, 34.2 / 33.2, 44.3 / 38.0, with roulette 8.41 / 8.56, 10.3 / 9.4, 13.0 / 12.2; media by
-// voxel 8.43 / 8.36, 11.7 / 10.6, 13.7 / 13.2; a replay into flux of 6763 and 22470 photons 4.96 / 4.93, 4.94 / 4.92.
 // Where even that leaves every warp of the full grid no more than four photons, the full grid: 1e4 photons, a warp's
 // spread over its lanes as below, 1.35 / 1.30 / 1.23 on the cube, 1.54 / 1.51 / 1.49 with detectors (3e4: 1.49 / 1.53 / 1.68).
 int transport_grid(const KParams& p, bool savedet, unsigned per_thread, int grid, int block, int sms, unsigned long long n) {

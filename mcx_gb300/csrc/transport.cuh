@@ -213,7 +213,8 @@ constexpr size_t kSmemPerCta = 227 * 1024;      // shared memory a CTA may have 
 int transport_mode(const KParams& p, bool savedet);
 // Occupancy-derived CTAs per SM for the chosen variant.
 int transport_blocks_per_sm(bool reflect, bool savedet, int mode, int block, size_t smem_bytes);
-// CTAs to launch for n photons on their own streams, at most `grid` (whole CTAs on every one of `sms` SMs).
+// CTAs to launch for n photons on their own streams, about `per_thread` to a thread, at most `grid` (whole CTAs on every one
+// of `sms` SMs).
 int transport_grid(const KParams& p, bool savedet, unsigned per_thread, int grid, int block, int sms, unsigned long long n);
 // Lanes of a warp left without a photon in a run of n (KParams::spare), for a launch that has the GPU to itself.
 unsigned transport_spare(int grid, int block, unsigned long long n);
