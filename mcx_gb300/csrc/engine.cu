@@ -417,7 +417,8 @@ unsigned photons_a_thread(const Config* cfg, const KParams& k) {
     };
     if (label(-1.f)) return 1;
     uint32_t med = 0;
-    for (int s = 0; s <= k.nx + k.ny + k.nz + (int)k.maxvoidstep && !med; s++) med = label((float)s);
+    const int reach = k.nx + k.ny + k.nz + (int)std::min(std::max(k.maxvoidstep, 0.f), 10000.f);
+    for (int s = 0; s <= reach && !med; s++) med = label((float)s);
     if (!med) med = 1;          // the beam's axis misses the volume: of a wide source only
     if (med >= (uint32_t)k.medianum) return 1;
     const float4 m = k.prop[med];
