@@ -49,8 +49,8 @@ __device__ __forceinline__ uint64_t umma_desc_mn32(uint32_t saddr, uint32_t lbo,
 // the volume would meet is read as zeros.  A warp holds 16 output channels x three pairs x three dz; where there
 // are fewer such units than warps, they share a unit's K steps.  Bound by the copies, which nothing overlaps.  Rare, but a
 // training step that meets one infinity should not stall (GB300, us a call: finite, one infinity, X all NaN, and the
-// general kernel on any of them): 2 x 65^3 16 to 16 41, 197, 209, 113; 4 x 65^3 48 to 16 180, 913, 1180, 636; 4 x 33^3
-// 96 to 32 85, 722, 790, 176; 33^3 64 to 64 32, 198, 241, 49; 4 x 17^3 128 to 128 66, 960, 992, 76.  (A voxel at a time on the
+// general kernel on any of them): 2 x 65^3 16 to 16 41, 203, 219, 113; 4 x 65^3 48 to 16 181, 950, 1234, 636; 4 x 33^3
+// 96 to 32 86, 735, 804, 176; 33^3 64 to 64 33, 189, 227, 49; 4 x 17^3 128 to 128 67, 818, 847, 76.  (A voxel at a time on the
 // CUDA cores took 7.7 to 38 ms for one infinity and 14 to 110 for X all NaN.)
 template <int COUT>
 __device__ __noinline__ void wgrad_within(unsigned char* smem, const bf16* dy, const bf16* x, float* dw, const Geo& g, int cin, int tiles_x,
@@ -68,6 +68,8 @@ __device__ __noinline__ void wgrad_within(unsigned char* smem, const bf16* dy, c
         const int unit = (base + warp) / share, part = (base + warp) % share;
         const bool on = unit < units;
         const int mb = unit / trios, p0 = unit % trios * 3;
+        // the blocks of dY that this round's units hold: the others need not be copied
+        const int y_lo = base / share / trios * PZ * 256, y_hi = (min(units - 1, (base + WARPS - 1) / share) / trios + 1) * PZ * 256;
         float acc[3][3][2][4] = {};
         for (int t = t_lo; t < t_hi; ++t) {
             int r = t;
@@ -81,7 +83,7 @@ __device__ __noinline__ void wgrad_within(unsigned char* smem, const bf16* dy, c
                 return (unsigned)z < (unsigned)g.d && (unsigned)y < (unsigned)g.h && (unsigned)xx < (unsigned)g.w;
             };
             __syncthreads();        // the tile before has been read
-            for (int i = tid; i < S::YBYTES / 16; i += 32 * WARPS) {
+            for (int i = y_lo + tid; i < y_hi; i += 32 * WARPS) {
                 const int xx = x0 + (i >> 1) % 8, yy = y0 + (i >> 4) % 16, zz = z0 + (i >> 8) % PZ, c = (i >> 8) / PZ * 16 + (i & 1) * 8;
                 const bool in = within(zz, yy, xx);
                 cp_async16(smem_addr(sy + i), in ? dy + voxel(zz, yy, xx) * COUT + c : dy, in);
