@@ -68,7 +68,7 @@ __device__ __noinline__ void wgrad_within(unsigned char* smem, const bf16* dy, c
         const int unit = (base + warp) / share, part = (base + warp) % share;
         const bool on = unit < units;
         const int mb = unit / trios, p0 = unit % trios * 3;
-        // the blocks of dY that this round's units hold: the others need not be copied
+        // the blocks of dY that this pass's units hold: the others need not be copied
         const int y_lo = base / share / trios * PZ * 256, y_hi = (min(units - 1, (base + WARPS - 1) / share) / trios + 1) * PZ * 256;
         float acc[3][3][2][4] = {};
         for (int t = t_lo; t < t_hi; ++t) {
